@@ -90,117 +90,168 @@ struct EvalHView {
     const Fr* scale;
 };
 
-// max permutation columns whose beta delta^c factors are staged per block
+// max permutation columns whose beta delta^c factors, and gate-term
+// coefficients, are staged per block as known factors
 static constexpr int EVAL_H_MAX_PERM = 256;
+static constexpr int EVAL_H_MAX_TERMS = 128;
+// threads a block: four blocks of 128 an SM share 2^17 rows out as 6.9 blocks an
+// SM (7 at most), two of 256 as 3.5 (4 at most): 1.28 against 1.44 ms
+static constexpr int EH_TB = 128;
 
-__global__ void __launch_bounds__(256, 2) eval_h_fused_kernel(Fr* h, EvalHView a) {
+// The factors fixed for a launch, in known-factor form: beta and the powers
+// of y the sum over constraints needs.
+enum { EH_BETA, EH_Y, EH_Y2, EH_Y3, EH_YG, EH_Y0, EH_YL, EH_FACTORS };
+
+// h is the Horner sum in y over the constraints in their order.  Constraints
+// come multiplied by one of l_0, l_last and l_active, so the sum is kept as
+// one Horner accumulator for each of the three, multiplied by its Lagrange
+// value once at the end:
+//   h = y^SG gates + l_0 (y^S0 P_0 + y^2 A_0) + l_last (y^SL P_last + y A_last) + l_active A
+// with P_0 = 1 - z_0 and the chunk links, P_last = z_last^2 - z_last, A_0 and
+// A_last the lookups' and shuffles' first two constraints in y^3 (for lookups
+// both are z, so one accumulator serves both), A the chunk products in y and
+// then the third constraints in y^3.  A lookup costs two products by the known
+// y^3 and two full ones instead of three and five, a chunk link or product one
+// known product instead of one of each.  Bound by the multiply pipe (ncu: 75%
+// of its cycles at 13 warps an SM): at 2^17 rows of 17 gates, 60 permutation
+// columns, 24 lookups and 4 shuffles 1.28 ms, against 1.59 ms with every
+// constraint added to one accumulator.
+__global__ void __launch_bounds__(EH_TB, 512 / EH_TB) eval_h_fused_kernel(Fr* h, EvalHView a) {
     __shared__ KnownFr s_dbeta[EVAL_H_MAX_PERM];
+    __shared__ KnownFr s_coef[EVAL_H_MAX_TERMS];
+    __shared__ KnownFr s_k[EH_FACTORS];
     for (int c = threadIdx.x; c < a.perm_cols_n; c += blockDim.x) s_dbeta[c] = known_fr(ld_elem<FrCfg>(a.perm_dbeta + c));
-    const KnownFr ky = block_known(a.y);
+    const uint32_t triples = 3u * ((uint32_t)a.lookups + (uint32_t)a.shuffles);
+    const uint32_t ch = (uint32_t)a.perm_chunks;
+    if (threadIdx.x < EH_FACTORS) {
+        const int k = (int)threadIdx.x;
+        const uint32_t e = k == EH_Y    ? 1u
+                           : k == EH_Y2 ? 2u
+                           : k == EH_Y3 ? 3u
+                           : k == EH_YG ? (ch ? 2u * ch + 1u : 0u) + triples
+                           : k == EH_Y0 ? ch + triples
+                                        : (ch ? 2u * ch - 1u : 0u) + triples;
+        const Fr v = k == EH_BETA ? (a.beta ? ld_elem<FrCfg>(a.beta) : fe_zero<FrCfg>())
+                                  : fe_pow_u32<FrCfg>(fe_canon<FrCfg>(ld_elem<FrCfg>(a.y)), e);
+        s_k[k] = known_fr(v);
+    }
+    // a term starts at entry 0 and after every null, so starts are at least two
+    // entries apart and entry vi / 2 numbers them
+    for (int vi = threadIdx.x; vi < a.gate_terms_n && vi < 2 * EVAL_H_MAX_TERMS; vi += blockDim.x)
+        if (a.gate_terms[vi] && (vi == 0 || !a.gate_terms[vi - 1]))
+            s_coef[vi >> 1] = known_fr(ld_elem<FrCfg>(a.gate_terms[vi]));
+    __syncthreads();
     const Fr one = fe_one<FrCfg>();
     const Fr beta = a.beta ? fe_canon<FrCfg>(ld_elem<FrCfg>(a.beta)) : fe_zero<FrCfg>();
     const Fr gamma = a.gamma ? fe_canon<FrCfg>(ld_elem<FrCfg>(a.gamma)) : fe_zero<FrCfg>();
-    KnownFr kbeta = known_fr(beta);
     const uint32_t n = a.n;
     QZ_GRID_LOOP(i, n) {
         // gates: sum_t coeff_t prod_j col_tj[i + rot_tj]
-        Fr acc = fe_zero<FrCfg>();
+        Fr g = fe_zero<FrCfg>();
         {
             int vi = 0, ri = 0;
             while (vi < a.gate_terms_n) {
-                Fr t = ld_elem<FrCfg>(a.gate_terms[vi++]);
+                const int first = vi++;
+                Fr t;
+                if (vi < a.gate_terms_n && a.gate_terms[vi] && first < 2 * EVAL_H_MAX_TERMS) {
+                    t = mul_known(ld_elem<FrCfg>(a.gate_terms[vi] + rot_row(i, a.gate_rots[ri] * a.rot_scale, n)),
+                                  s_coef[first >> 1]);
+                    vi++;
+                    ri++;
+                } else {
+                    t = ld_elem<FrCfg>(a.gate_terms[first]);
+                }
                 while (vi < a.gate_terms_n && a.gate_terms[vi]) {
                     t = fe_mul_lazy<FrCfg>(t, ld_elem<FrCfg>(a.gate_terms[vi] +
                                                              rot_row(i, a.gate_rots[ri] * a.rot_scale, n)));
                     vi++;
                     ri++;
                 }
-                acc = fe_add_lazy<FrCfg>(acc, t);
+                g = fe_add_lazy<FrCfg>(g, t);
                 vi++;
             }
         }
-        const Fr l0 = ld_elem<FrCfg>(a.l0 + i);
-        const Fr ll = ld_elem<FrCfg>(a.l_last + i);
-        const Fr la = ld_elem<FrCfg>(a.l_active + i);
-        if (a.perm_chunks > 0) {
-            // l_0 (1 - z_0) and l_last (z_last^2 - z_last) (cuda/bn254.cu:664-699)
-            const Fr z0 = ld_elem<FrCfg>(a.perm_z[0] + i);
-            const Fr zl = ld_elem<FrCfg>(a.perm_z[a.perm_chunks - 1] + i);
-            acc = mul_known(acc, ky);
-            acc = fe_add_lazy<FrCfg>(acc, fe_mul_lazy<FrCfg>(l0, fe_sub_lazy<FrCfg>(one, z0)));
-            acc = mul_known(acc, ky);
-            acc = fe_add_lazy<FrCfg>(acc, fe_mul_lazy<FrCfg>(ll, fe_sub_lazy<FrCfg>(fe_mul_lazy<FrCfg>(zl, zl), zl)));
+        if (ch || triples) g = mul_known(g, s_k[EH_YG]);
+        const uint32_t rn = rot_row(i, a.rot_scale, n);
+        Fr act = fe_zero<FrCfg>();  // A
+        Fr p0 = act, pl = act;      // y^S0 P_0, y^SL P_last
+        if (ch) {
+            // l_0 (1 - z_0) and l_last (z_last^2 - z_last) (cuda/bn254.cu:664-699),
             // chunk links l_0 (z_j - z_{j-1}(w^last X)) (cuda/bn254.cu:701-733)
+            const Fr zl = ld_elem<FrCfg>(a.perm_z[ch - 1] + i);
+            pl = mul_known(fe_sub_lazy<FrCfg>(fe_mul_lazy<FrCfg>(zl, zl), zl), s_k[EH_YL]);
+            p0 = mul_known(fe_sub_lazy<FrCfg>(one, ld_elem<FrCfg>(a.perm_z[0] + i)), s_k[EH_Y]);
             const uint32_t rp = rot_row(i, a.perm_last_rot * a.rot_scale, n);
-            for (int j = 1; j < a.perm_chunks; j++) {
-                acc = mul_known(acc, ky);
-                const Fr d = fe_sub_lazy<FrCfg>(ld_elem<FrCfg>(a.perm_z[j] + i), ld_elem<FrCfg>(a.perm_z[j - 1] + rp));
-                acc = fe_add_lazy<FrCfg>(acc, fe_mul_lazy<FrCfg>(d, l0));
-            }
+            for (uint32_t j = 1; j < ch; j++)
+                p0 = fe_add_lazy<FrCfg>(
+                    mul_known(p0, s_k[EH_Y]),
+                    fe_sub_lazy<FrCfg>(ld_elem<FrCfg>(a.perm_z[j] + i), ld_elem<FrCfg>(a.perm_z[j - 1] + rp)));
+            p0 = mul_known(p0, s_k[EH_Y0]);
             // l_active (z(wX) prod (v + beta sigma + gamma) - z(X) prod (v + beta delta^c X + gamma))
             // (src/eval_h.rs:700-810)
             const Fr X = ld_elem<FrCfg>(a.x + i);
-            const uint32_t rn = rot_row(i, a.rot_scale, n);
             int c = 0;
-            for (int j = 0; j < a.perm_chunks; j++) {
+            for (uint32_t j = 0; j < ch; j++) {
                 Fr L = ld_elem<FrCfg>(a.perm_z[j] + rn);
                 Fr R = ld_elem<FrCfg>(a.perm_z[j] + i);
                 const int end = c + a.perm_chunk_len < a.perm_cols_n ? c + a.perm_chunk_len : a.perm_cols_n;
                 for (; c < end; c++) {
                     const Fr v = fe_add_lazy<FrCfg>(ld_elem<FrCfg>(a.perm_cols[c] + i), gamma);
-                    const Fr bs = mul_known(ld_elem<FrCfg>(a.perm_sigmas[c] + i), kbeta);
+                    const Fr bs = mul_known(ld_elem<FrCfg>(a.perm_sigmas[c] + i), s_k[EH_BETA]);
                     L = fe_mul_lazy<FrCfg>(L, fe_add_lazy<FrCfg>(v, bs));
                     R = fe_mul_lazy<FrCfg>(R, fe_add_lazy<FrCfg>(v, mul_known(X, s_dbeta[c])));
                 }
-                acc = mul_known(acc, ky);
-                acc = fe_add_lazy<FrCfg>(acc, fe_mul_lazy<FrCfg>(la, fe_sub_lazy<FrCfg>(L, R)));
+                if (j) act = mul_known(act, s_k[EH_Y]);
+                act = fe_add_lazy<FrCfg>(act, fe_sub_lazy<FrCfg>(L, R));
             }
         }
         // logup lookups with one input per set (cuda/bn254.cu:867-921): with
         // f' = input + beta, t' = table + beta,
         // y^3 acc + y^2 l_0 z + y l_last z + l_active (((z(wX) - z) t' + m) f' - t')
+        Fr a0 = fe_zero<FrCfg>();  // A_0 (and A_last while only lookups have been added)
         for (int k = 0; k < a.lookups; k++) {
             const Fr* const* q = a.lookup_cols + 4 * k;
-            const Fr fb = fe_add_lazy<FrCfg>(ld_elem<FrCfg>(q[0] + i), beta);
             const Fr tb = fe_add_lazy<FrCfg>(ld_elem<FrCfg>(q[1] + i), beta);
-            const Fr m = ld_elem<FrCfg>(q[2] + i);
             const Fr z = ld_elem<FrCfg>(q[3] + i);
-            const Fr zn = ld_elem<FrCfg>(q[3] + rot_row(i, a.rot_scale, n));
-            acc = mul_known(acc, ky);
-            acc = fe_add_lazy<FrCfg>(acc, fe_mul_lazy<FrCfg>(l0, z));
-            acc = mul_known(acc, ky);
-            acc = fe_add_lazy<FrCfg>(acc, fe_mul_lazy<FrCfg>(ll, z));
-            acc = mul_known(acc, ky);
-            Fr u = fe_mul_lazy<FrCfg>(fe_sub_lazy<FrCfg>(zn, z), tb);
-            u = fe_mul_lazy<FrCfg>(fe_add_lazy<FrCfg>(u, m), fb);
-            u = fe_sub_lazy<FrCfg>(u, tb);
-            acc = fe_add_lazy<FrCfg>(acc, fe_mul_lazy<FrCfg>(u, la));
+            Fr u = fe_mul_lazy<FrCfg>(fe_sub_lazy<FrCfg>(ld_elem<FrCfg>(q[3] + rn), z), tb);
+            u = fe_add_lazy<FrCfg>(u, ld_elem<FrCfg>(q[2] + i));
+            u = fe_mul_lazy<FrCfg>(u, fe_add_lazy<FrCfg>(ld_elem<FrCfg>(q[0] + i), beta));
+            act = fe_add_lazy<FrCfg>(mul_known(act, s_k[EH_Y3]), fe_sub_lazy<FrCfg>(u, tb));
+            a0 = fe_add_lazy<FrCfg>(k ? mul_known(a0, s_k[EH_Y3]) : a0, z);
         }
         // shuffles (cuda/bn254.cu:1017-1071): with l = prod (input_g + beta_g),
         // r = prod (table_g + beta_g),
         // y^3 acc + y^2 l_0 (1 - z) + y l_last (z^2 - z) + l_active (r z(wX) - l z)
+        Fr al = a0;
         {
             int off = 0;
             for (int s = 0; s < a.shuffles; s++) {
                 const Fr* const* q = a.shuffle_cols + off;
-                const int g = a.shuffle_group_len[s];
+                const int gl = a.shuffle_group_len[s];
                 const Fr z = ld_elem<FrCfg>(q[0] + i);
-                const Fr zn = ld_elem<FrCfg>(q[0] + rot_row(i, a.rot_scale, n));
-                Fr l = one, r = one;
-                for (int t = 0; t < g; t++) {
+                // the products start from z(wX) and z
+                Fr l = z, r = ld_elem<FrCfg>(q[0] + rn);
+                for (int t = 0; t < gl; t++) {
                     const Fr bt = ld_elem<FrCfg>(a.shuffle_betas + t);
                     l = fe_mul_lazy<FrCfg>(l, fe_add_lazy<FrCfg>(ld_elem<FrCfg>(q[1 + 2 * t] + i), bt));
                     r = fe_mul_lazy<FrCfg>(r, fe_add_lazy<FrCfg>(ld_elem<FrCfg>(q[2 + 2 * t] + i), bt));
                 }
-                acc = mul_known(acc, ky);
-                acc = fe_add_lazy<FrCfg>(acc, fe_mul_lazy<FrCfg>(l0, fe_sub_lazy<FrCfg>(one, z)));
-                acc = mul_known(acc, ky);
-                acc = fe_add_lazy<FrCfg>(acc, fe_mul_lazy<FrCfg>(ll, fe_sub_lazy<FrCfg>(fe_mul_lazy<FrCfg>(z, z), z)));
-                acc = mul_known(acc, ky);
-                const Fr u = fe_sub_lazy<FrCfg>(fe_mul_lazy<FrCfg>(r, zn), fe_mul_lazy<FrCfg>(l, z));
-                acc = fe_add_lazy<FrCfg>(acc, fe_mul_lazy<FrCfg>(u, la));
-                off += 1 + 2 * g;
+                act = fe_add_lazy<FrCfg>(mul_known(act, s_k[EH_Y3]), fe_sub_lazy<FrCfg>(r, l));
+                a0 = fe_add_lazy<FrCfg>(mul_known(a0, s_k[EH_Y3]), fe_sub_lazy<FrCfg>(one, z));
+                al = fe_add_lazy<FrCfg>(mul_known(al, s_k[EH_Y3]),
+                                        fe_sub_lazy<FrCfg>(fe_mul_lazy<FrCfg>(z, z), z));
+                off += 1 + 2 * gl;
             }
+        }
+        Fr acc = g;
+        if (ch || triples) {
+            if (triples) {
+                p0 = fe_add_lazy<FrCfg>(p0, mul_known(a0, s_k[EH_Y2]));
+                pl = fe_add_lazy<FrCfg>(pl, mul_known(al, s_k[EH_Y]));
+            }
+            acc = fe_add_lazy<FrCfg>(acc, fe_mul_lazy<FrCfg>(p0, ld_elem<FrCfg>(a.l0 + i)));
+            acc = fe_add_lazy<FrCfg>(acc, fe_mul_lazy<FrCfg>(pl, ld_elem<FrCfg>(a.l_last + i)));
+            acc = fe_add_lazy<FrCfg>(acc, fe_mul_lazy<FrCfg>(act, ld_elem<FrCfg>(a.l_active + i)));
         }
         if (a.scale) acc = fe_mul_lazy<FrCfg>(acc, ld_elem<FrCfg>(a.scale));
         st_elem<FrCfg>(h + i, fe_canon<FrCfg>(acc));
@@ -377,7 +428,7 @@ cudaError_t zkp_eval_h_fused(void* h, const zkp_eval_h_args* args, cudaStream_t 
     v.shuffle_group_len = reinterpret_cast<const int*>(g.shuffle_group_len);
     v.shuffle_betas = CFr(g.shuffle_betas);
     v.scale = CFr(g.scale);
-    eval_h_fused_kernel<<<qz_grid(n, 256), 256, 0, stream>>>(reinterpret_cast<Fr*>(h), v);
+    eval_h_fused_kernel<<<qz_grid(n, EH_TB), EH_TB, 0, stream>>>(reinterpret_cast<Fr*>(h), v);
     return cudaGetLastError();
 }
 
