@@ -86,6 +86,8 @@ struct MsmScratch {
     Aff* phi;            // n endomorphism images of the bases (GLV plans without a table), else null
 };
 
+// buckets a reduction segment sums, for NB buckets in sets of B
+uint32_t msm_reduce_segment(uint64_t NB, uint32_t B, uint32_t max_threads);
 MsmPlan msm_make_plan(uint32_t n, int c, bool glv = true);
 // plan over a table of pre-multiplied bases (msm_table_*): all windows share
 // one bucket set; the table holds nsrs >= n points per window

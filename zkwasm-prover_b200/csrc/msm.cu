@@ -11,9 +11,10 @@
 //               that cross a slice boundary are left as head / tail partials
 //   5. merge    partials of buckets split across slices: a reduction by key,
 //               warp-segmented scans level by level (log-depth in the split)
-//   6. reduce   per window, segments of buckets by running sums:
-//               sum_b (b+1) B_b = S_seg + lo * T_seg
-//   7. window   tree sum of the segment results per window
+//   6. reduce   per window, sum_b (b+1) B_b: segments of buckets by running
+//               sums, then one tree that leaves a sum per bit of the segment
+//               number (msm_common.cuh)
+//   7. window   Horner over those bits per window
 //   8. final    Horner over windows (c doublings each) -> Jacobian output,
 //               four warps evaluating the independent products of each formula
 //
@@ -374,54 +375,30 @@ static cudaError_t msm_merge(uint32_t* part_key, Xyzz* part_pt, uint32_t nacc, X
     return cudaSuccess;
 }
 
-// Thread t = w G + g sums segment g of window w by running sums; then each
-// group of GS = min(G, 128) consecutive threads (one window) adds its results
-// as a tree, and the group's sum goes to segsum[t / GS], so the window
-// kernel is left with G / GS partial sums per window.
-__global__ void __launch_bounds__(128) msm_reduce_kernel(const Xyzz* __restrict__ buckets,
-                                                         const uint32_t* __restrict__ offset, int W, uint32_t B,
-                                                         uint32_t seg, uint32_t G, Xyzz* __restrict__ segsum) {
-    __shared__ Xyzz sm[128];
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    Xyzz S = xyzz_identity();
-    if (t < (uint32_t)W * G) {
-        const uint32_t w = t / G, g = t % G;
-        const uint32_t lo = g * seg;
-        Xyzz T = xyzz_identity();
-        for (uint32_t j = 0; j < seg; j++) {
-            const uint32_t b = lo + seg - 1 - j;
-            const uint32_t key = w * B + b;
-            if (offset[key + 1] != offset[key]) T = xyzz_add(T, ld_xyzz(buckets + key));
-            S = xyzz_add(S, T);
-        }
-        if (lo) S = xyzz_add(S, xyzz_mul_u32(T, lo));
-    }
-    const uint32_t GS = G < 128 ? G : 128;
-    const uint32_t k = threadIdx.x;
-    sm[k] = S;
-    __syncthreads();
-    for (uint32_t h = GS >> 1; h > 0; h >>= 1) {
-        if ((k & (GS - 1)) < h) sm[k] = xyzz_add(sm[k], sm[k + h]);
-        __syncthreads();
-    }
-    if ((k & (GS - 1)) == 0 && t < (uint32_t)W * G) st_xyzz(segsum + t / GS, sm[k]);
+// Bucket reduction (msm_common.cuh): thread t = w G + g takes segment g of set w
+__global__ void __launch_bounds__(RED_T) msm_reduce_kernel(const Xyzz* __restrict__ buckets,
+                                                           const uint32_t* __restrict__ offset, uint32_t sets,
+                                                           uint32_t B, uint32_t seg, uint32_t G,
+                                                           Xyzz* __restrict__ segsum) {
+    __shared__ Xyzz Tp[RED_T], Sp[RED_T];
+    const uint32_t t = blockIdx.x * RED_T + threadIdx.x;
+    const uint32_t w = t / G, g = t % G;
+    const bool live = w < sets;
+    Xyzz S = xyzz_identity(), T = S;
+    if (live) red_segment(buckets, offset, w * B + g * seg, seg, S, T);
+    red_groups(Tp, Sp, S, T, G, live, segsum + (size_t)w * G, g / RED_T);
 }
 
-// one CTA per window; blockDim (a power of two, <= G) threads first add
-// G / blockDim segment results each, then reduce as a tree
-__global__ void __launch_bounds__(256) msm_window_kernel(const Xyzz* __restrict__ segsum, uint32_t G, Xyzz* __restrict__ winsum) {
-    extern __shared__ uint4 smem_u4[];
-    Xyzz* sm = reinterpret_cast<Xyzz*>(smem_u4);
-    const uint32_t w = blockIdx.x, i = threadIdx.x, T = blockDim.x;
-    Xyzz acc = ld_xyzz(segsum + (size_t)w * G + i);
-    for (uint32_t k = i + T; k < G; k += T) acc = xyzz_add(acc, ld_xyzz(segsum + (size_t)w * G + k));
-    sm[i] = acc;
-    __syncthreads();
-    for (uint32_t h = T >> 1; h > 0; h >>= 1) {
-        if (i < h) sm[i] = xyzz_add(sm[i], sm[i + h]);
-        __syncthreads();
-    }
-    if (i == 0) st_xyzz(winsum + w, sm[0]);
+__global__ void __launch_bounds__(RED_T) msm_plane_kernel(Xyzz* segsum, uint32_t G) {
+    __shared__ Xyzz sm[RED_T];
+    red_plane(sm, segsum + (size_t)blockIdx.x * G, G / RED_T, blockIdx.y);
+}
+
+__global__ void __launch_bounds__(COOP_THREADS) msm_window_kernel(const Xyzz* __restrict__ segsum, uint32_t G,
+                                                                  uint32_t seg, Xyzz* __restrict__ winsum) {
+    __shared__ Fq buf[8];
+    const Xyzz r = red_horner(buf, segsum + (size_t)blockIdx.x * G, G, seg);
+    if (threadIdx.x == 0) st_xyzz(winsum + blockIdx.x, r);
 }
 
 // one CTA of COOP_THREADS threads
@@ -569,6 +546,18 @@ int msm_batch_table_default_window(const uint32_t* n, uint32_t count) {
     return best;
 }
 
+// Buckets a reduction segment sums (a power of two) when a launch reduces NB
+// buckets in all, in sets of B: a segment of s buckets costs 2 (s - 1)
+// additions one after the other, a group's tree 14 warp additions whatever s
+// is, so segments are as long as leaves every SM two blocks of 128 segments;
+// and long enough for max_threads segments in all (the scratch they are kept
+// in) and RED_MAX_G a set.
+uint32_t msm_reduce_segment(uint64_t NB, uint32_t B, uint32_t max_threads) {
+    uint32_t s = 1;
+    while (s < B && (NB / s > max_threads || B / s > RED_MAX_G || NB / (2 * (uint64_t)s) >= 2ull * 148 * RED_T)) s *= 2;
+    return s;
+}
+
 static void plan_finish(MsmPlan& p) {
     p.B = 1u << (p.c - 1);
     p.NB = (uint32_t)p.Wb * p.B;
@@ -579,14 +568,8 @@ static void plan_finish(MsmPlan& p) {
     p.L = (uint32_t)L;
     p.nacc = (uint32_t)((max_entries + L - 1) / L);
     if (p.nacc == 0) p.nacc = 1;
-    // up to ZK_MSM_REDUCE_THREADS reduction threads in total (the running-sum
-    // segments are latency bound, so they need many threads), at most 4096 per
-    // window when there is one bucket set per window
-    const uint32_t gcap = p.Wb == 1 ? ZK_MSM_REDUCE_THREADS : 4096;
-    uint32_t G = 1;
-    while (G < gcap && (uint64_t)G * 2 * p.Wb <= ZK_MSM_REDUCE_THREADS && G * 2 <= p.B) G *= 2;
-    p.G = G;
-    p.seg = p.B / G;
+    p.seg = msm_reduce_segment(p.NB, p.B, ZK_MSM_REDUCE_THREADS);
+    p.G = p.B / p.seg;
 }
 
 MsmPlan msm_make_plan(uint32_t n, int c, bool glv) {
@@ -817,12 +800,14 @@ cudaError_t msm_run(Jac* out, const Aff* bases, const Fr* scalars, const MsmPlan
     ZK_CHECK(cudaGetLastError());
     ZK_CHECK(msm_merge(s.part_key, s.part_pt, p.nacc, s.buckets, st));
     const uint32_t nred = (uint32_t)p.Wb * p.G;
-    msm_reduce_kernel<<<(nred + 127) / 128, 128, 0, st>>>(s.buckets, s.offset, p.Wb, p.B, p.seg, p.G, s.segsum);
+    msm_reduce_kernel<<<(nred + RED_T - 1) / RED_T, RED_T, 0, st>>>(s.buckets, s.offset, p.Wb, p.B, p.seg, p.G,
+                                                                    s.segsum);
     ZK_CHECK(cudaGetLastError());
-    // partial sums per window left by the reduce kernel's group trees
-    const uint32_t parts = p.G < 128 ? 1u : p.G / 128u;
-    const uint32_t wt = parts < 256 ? parts : 256;
-    msm_window_kernel<<<p.Wb, wt, (size_t)wt * sizeof(Xyzz), st>>>(s.segsum, parts, s.winsum);
+    if (p.G > RED_T) {
+        msm_plane_kernel<<<dim3(p.Wb, RED_PLANES), RED_T, 0, st>>>(s.segsum, p.G);
+        ZK_CHECK(cudaGetLastError());
+    }
+    msm_window_kernel<<<p.Wb, COOP_THREADS, 0, st>>>(s.segsum, p.G, p.seg, s.winsum);
     ZK_CHECK(cudaGetLastError());
     if (park_note) {
         msm_park_kernel<<<1, 1, 0, st>>>(reinterpret_cast<MsmParked*>(park_note), (uint32_t)p.Wb, (uint32_t)p.c,

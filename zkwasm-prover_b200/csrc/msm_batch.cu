@@ -124,59 +124,36 @@ __global__ void batch_scatter_kernel(const BatchDesc* d, uint32_t count, const F
     }
 }
 
-// as msm_reduce_kernel, over every MSM's (window, segment) threads; each
-// MSM's threads start on a 128-thread boundary, so a CTA serves one MSM and
-// its group trees (GS = min(G, 128) threads, one window) stay inside the CTA
-__global__ void __launch_bounds__(128) batch_reduce_kernel(const BatchDesc* d, uint32_t count, uint32_t total,
-                                                           const Xyzz* buckets, const uint32_t* offset,
-                                                           Xyzz* segsum) {
-    __shared__ Xyzz sm[128];
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t i = find_desc<&BatchDesc::red_off>(d, count, blockIdx.x * blockDim.x);
-    const BatchDesc q = d[i];
-    const uint32_t lt = t - q.red_off;
-    Xyzz S = xyzz_identity();
-    if (t < total && lt < q.Wb * q.G) {
-        const uint32_t w = lt / q.G, g = lt % q.G;
-        const uint32_t lo = g * q.seg;
-        Xyzz T = xyzz_identity();
-        for (uint32_t j = 0; j < q.seg; j++) {
-            const uint32_t key = q.key_off + w * q.B + lo + q.seg - 1 - j;
-            if (offset[key + 1] != offset[key]) T = xyzz_add(T, ld_xyzz(buckets + key));
-            S = xyzz_add(S, T);
-        }
-        if (lo) S = xyzz_add(S, xyzz_mul_u32(T, lo));
-    }
-    const uint32_t GS = q.G < 128 ? q.G : 128;
-    const uint32_t k = threadIdx.x;
-    sm[k] = S;
-    __syncthreads();
-    for (uint32_t h = GS >> 1; h > 0; h >>= 1) {
-        if ((k & (GS - 1)) < h) sm[k] = xyzz_add(sm[k], sm[k + h]);
-        __syncthreads();
-    }
-    if ((k & (GS - 1)) == 0 && t < total && lt < q.Wb * q.G) st_xyzz(segsum + q.red_off + lt / GS, sm[k]);
+// as msm_reduce_kernel, over every MSM's (set, segment) threads; each MSM's
+// threads start on a RED_T boundary, so a CTA serves one MSM and its groups
+// (min(G, RED_T) threads of one set) stay inside the CTA
+__global__ void __launch_bounds__(RED_T) batch_reduce_kernel(const BatchDesc* d, uint32_t count, const Xyzz* buckets,
+                                                             const uint32_t* offset, Xyzz* segsum) {
+    __shared__ Xyzz Tp[RED_T], Sp[RED_T];
+    const uint32_t t = blockIdx.x * RED_T + threadIdx.x;
+    const BatchDesc q = d[find_desc<&BatchDesc::red_off>(d, count, blockIdx.x * RED_T)];
+    const uint32_t lt = t - q.red_off, w = lt / q.G, g = lt % q.G;
+    const bool live = w < q.Wb;
+    Xyzz S = xyzz_identity(), T = S;
+    if (live) red_segment(buckets, offset, q.key_off + w * q.B + g * q.seg, q.seg, S, T);
+    red_groups(Tp, Sp, S, T, q.G, live, segsum + q.red_off + (size_t)w * q.G, g / RED_T);
 }
 
-// one CTA per (MSM, bucket set): adds the set's G / min(G, 128) group sums,
-// each thread a strided subset first, then a tree (blockDim a power of two)
-__global__ void __launch_bounds__(256) batch_window_kernel(const BatchDesc* d, uint32_t count, const Xyzz* segsum, Xyzz* winsum) {
-    extern __shared__ uint4 smem_u4[];
-    Xyzz* sm = reinterpret_cast<Xyzz*>(smem_u4);
-    const uint32_t b = blockIdx.x, k = threadIdx.x;
-    const uint32_t i = find_desc<&BatchDesc::win_off>(d, count, b);
-    const BatchDesc q = d[i];
-    const uint32_t w = b - q.win_off;
-    const uint32_t parts = q.G < 128 ? 1u : q.G / 128u;
-    Xyzz acc = xyzz_identity();
-    for (uint32_t g = k; g < parts; g += blockDim.x) acc = xyzz_add(acc, ld_xyzz(segsum + q.red_off + w * parts + g));
-    sm[k] = acc;
-    __syncthreads();
-    for (uint32_t h = blockDim.x >> 1; h > 0; h >>= 1) {
-        if (k < h) sm[k] = xyzz_add(sm[k], sm[k + h]);
-        __syncthreads();
-    }
-    if (k == 0) st_xyzz(winsum + b, sm[0]);
+// block (set, plane), sets of one group excepted
+__global__ void __launch_bounds__(RED_T) batch_plane_kernel(const BatchDesc* d, uint32_t count, Xyzz* segsum) {
+    __shared__ Xyzz sm[RED_T];
+    const BatchDesc q = d[find_desc<&BatchDesc::win_off>(d, count, blockIdx.x)];
+    if (q.G <= RED_T) return;  // uniform: stage 1 left the set's planes
+    red_plane(sm, segsum + q.red_off + (size_t)(blockIdx.x - q.win_off) * q.G, q.G / RED_T, blockIdx.y);
+}
+
+// one CTA per set
+__global__ void __launch_bounds__(COOP_THREADS) batch_window_kernel(const BatchDesc* d, uint32_t count,
+                                                                    const Xyzz* segsum, Xyzz* winsum) {
+    __shared__ Fq buf[8];
+    const BatchDesc q = d[find_desc<&BatchDesc::win_off>(d, count, blockIdx.x)];
+    const Xyzz r = red_horner(buf, segsum + q.red_off + (size_t)(blockIdx.x - q.win_off) * q.G, q.G, q.seg);
+    if (threadIdx.x == 0) st_xyzz(winsum + blockIdx.x, r);
 }
 
 // one CTA of COOP_THREADS threads per MSM
@@ -222,7 +199,7 @@ static size_t al(size_t x) { return (x + 255) / 256 * 256; }
 #ifndef ZK_MSM_BATCH_REDUCE_THREADS
 #define ZK_MSM_BATCH_REDUCE_THREADS 131072
 #endif
-static constexpr uint64_t BATCH_REDUCE_THREADS = ZK_MSM_BATCH_REDUCE_THREADS;
+static constexpr uint32_t BATCH_REDUCE_THREADS = ZK_MSM_BATCH_REDUCE_THREADS;
 
 // nsrs > 0: every MSM runs over one table of pre-multiplied bases of width
 // c[0] (one bucket set per MSM); otherwise per-MSM widths c[i] (0 or a null c:
@@ -236,17 +213,11 @@ static bool batch_plan(const uint32_t* n, const int* c, uint32_t count, uint32_t
         plans[i] = nsrs ? msm_make_table_plan(n[i], c[0], nsrs) : msm_make_plan(n[i], c ? c[i] : 0, true);
         all_buckets += (uint64_t)plans[i].Wb * plans[i].B;
     }
-    // The reduction threads of the whole batch share one budget, in
-    // proportion to each MSM's buckets: a segment's closing product lo * T
-    // costs about 1.5 c additions, so many MSMs with the single-MSM thread
-    // counts would spend more on those than on the running sums themselves.
+    // the reduction's segments are sized for the buckets of the whole batch
     for (uint32_t i = 0; i < count; i++) {
         MsmPlan& p = plans[i];
-        const uint64_t share = BATCH_REDUCE_THREADS * (uint64_t)p.Wb * p.B / (all_buckets ? all_buckets : 1);
-        uint32_t G = 1;
-        while ((uint64_t)G * 2 * p.Wb <= share && G * 2 <= p.G) G *= 2;
-        p.G = G;
-        p.seg = p.B / G;
+        p.seg = msm_reduce_segment(all_buckets, p.B, BATCH_REDUCE_THREADS);
+        p.G = p.B / p.seg;
     }
     uint64_t key = 0, sc = 0, red = 0, win = 0, ent = 0;
     for (uint32_t i = 0; i < count; i++) {
@@ -365,14 +336,13 @@ cudaError_t msm_batch_run(Jac* out, const Aff* bases, const Fr* const* scalars, 
         ZK_CHECK(
             msm_accumulate_merge(entries, offset, L.NB, bases, phi, L.nmax, L.L, L.nacc, buckets, pkey, ppt, st));
     }
-    batch_reduce_kernel<<<(L.red_total + 127) / 128, 128, 0, st>>>(d, count, L.red_total, buckets, offset, segsum);
+    batch_reduce_kernel<<<L.red_total / RED_T, RED_T, 0, st>>>(d, count, buckets, offset, segsum);
     ZK_CHECK(cudaGetLastError());
-    const uint32_t max_parts = L.maxG < 128 ? 1u : L.maxG / 128u;
-    uint32_t bd = 1;
-    while (bd < max_parts && bd < 256) bd <<= 1;
-    static SmemOptIn opt;
-    ZK_CHECK(opt.ensure(batch_window_kernel, 512 * (int)sizeof(Xyzz)));
-    batch_window_kernel<<<L.win_total, bd, (size_t)bd * sizeof(Xyzz), st>>>(d, count, segsum, winsum);
+    if (L.maxG > RED_T) {
+        batch_plane_kernel<<<dim3(L.win_total, RED_PLANES), RED_T, 0, st>>>(d, count, segsum);
+        ZK_CHECK(cudaGetLastError());
+    }
+    batch_window_kernel<<<L.win_total, COOP_THREADS, 0, st>>>(d, count, segsum, winsum);
     ZK_CHECK(cudaGetLastError());
     batch_final_kernel<<<count, COOP_THREADS, 0, st>>>(d, winsum, out);
     return cudaGetLastError();
