@@ -16,7 +16,7 @@
 //               number (msm_common.cuh)
 //   7. window   Horner over those bits per window
 //   8. final    Horner over windows (c doublings each) -> Jacobian output,
-//               four warps evaluating the independent products of each formula
+//               quads of lanes evaluating the independent products of each formula
 //
 // Reference behaviour replaced: cuda/msm.cu:9-467 (unsigned digits, CUB radix
 // sort, Jacobian accumulation, one-thread window combine) behind the C entry
@@ -376,7 +376,7 @@ static cudaError_t msm_merge(uint32_t* part_key, Xyzz* part_pt, uint32_t nacc, X
 }
 
 // Bucket reduction (msm_common.cuh): thread t = w G + g takes segment g of set w
-__global__ void __launch_bounds__(RED_T) msm_reduce_kernel(const Xyzz* __restrict__ buckets,
+__global__ void __launch_bounds__(RED_T, 2) msm_reduce_kernel(const Xyzz* __restrict__ buckets,
                                                            const uint32_t* __restrict__ offset, uint32_t sets,
                                                            uint32_t B, uint32_t seg, uint32_t G,
                                                            Xyzz* __restrict__ segsum) {
@@ -396,16 +396,14 @@ __global__ void __launch_bounds__(RED_T) msm_plane_kernel(Xyzz* segsum, uint32_t
 
 __global__ void __launch_bounds__(COOP_THREADS) msm_window_kernel(const Xyzz* __restrict__ segsum, uint32_t G,
                                                                   uint32_t seg, Xyzz* __restrict__ winsum) {
-    __shared__ Fq buf[8];
-    const Xyzz r = red_horner(buf, segsum + (size_t)blockIdx.x * G, G, seg);
-    if (threadIdx.x == 0) st_xyzz(winsum + blockIdx.x, r);
+    const Fq r = red_horner(segsum + (size_t)blockIdx.x * G, G, seg);
+    if (threadIdx.x < 4) qd_store(winsum + blockIdx.x, r);
 }
 
 // one CTA of COOP_THREADS threads
 __global__ void __launch_bounds__(COOP_THREADS) msm_final_kernel(const Xyzz* __restrict__ winsum, int W, int c,
                                                                   Jac* __restrict__ out) {
-    __shared__ Fq buf[8];
-    const Jac j = coop_horner(buf, winsum, W, c);
+    const Jac j = coop_horner(winsum, W, c);
     if (threadIdx.x == 0) {
         st_elem<FqCfg>(&out->x, j.x);
         st_elem<FqCfg>(&out->y, j.y);
@@ -740,11 +738,10 @@ __global__ void msm_park_kernel(MsmParked* note, uint32_t W, uint32_t c, const X
 // one CTA per region: regions[i] + note_off holds the note, the Jacobian
 // result goes to regions[i][0]
 __global__ void __launch_bounds__(COOP_THREADS) msm_collect_kernel(char* const* regions, uint32_t note_off) {
-    __shared__ Fq buf[8];
     char* base = regions[blockIdx.x];
     const MsmParked note = *reinterpret_cast<const MsmParked*>(base + note_off);
     if (note.magic != PARK_MAGIC) return;  // uniform: no msm() result parked here
-    const Jac j = coop_horner(buf, note.winsum, (int)note.W, (int)note.c);
+    const Jac j = coop_horner(note.winsum, (int)note.W, (int)note.c);
     if (threadIdx.x == 0) {
         Jac* out = reinterpret_cast<Jac*>(base);
         st_elem<FqCfg>(&out->x, j.x);

@@ -127,7 +127,7 @@ __global__ void batch_scatter_kernel(const BatchDesc* d, uint32_t count, const F
 // as msm_reduce_kernel, over every MSM's (set, segment) threads; each MSM's
 // threads start on a RED_T boundary, so a CTA serves one MSM and its groups
 // (min(G, RED_T) threads of one set) stay inside the CTA
-__global__ void __launch_bounds__(RED_T) batch_reduce_kernel(const BatchDesc* d, uint32_t count, const Xyzz* buckets,
+__global__ void __launch_bounds__(RED_T, 2) batch_reduce_kernel(const BatchDesc* d, uint32_t count, const Xyzz* buckets,
                                                              const uint32_t* offset, Xyzz* segsum) {
     __shared__ Xyzz Tp[RED_T], Sp[RED_T];
     const uint32_t t = blockIdx.x * RED_T + threadIdx.x;
@@ -150,19 +150,17 @@ __global__ void __launch_bounds__(RED_T) batch_plane_kernel(const BatchDesc* d, 
 // one CTA per set
 __global__ void __launch_bounds__(COOP_THREADS) batch_window_kernel(const BatchDesc* d, uint32_t count,
                                                                     const Xyzz* segsum, Xyzz* winsum) {
-    __shared__ Fq buf[8];
     const BatchDesc q = d[find_desc<&BatchDesc::win_off>(d, count, blockIdx.x)];
-    const Xyzz r = red_horner(buf, segsum + q.red_off + (size_t)(blockIdx.x - q.win_off) * q.G, q.G, q.seg);
-    if (threadIdx.x == 0) st_xyzz(winsum + blockIdx.x, r);
+    const Fq r = red_horner(segsum + q.red_off + (size_t)(blockIdx.x - q.win_off) * q.G, q.G, q.seg);
+    if (threadIdx.x < 4) qd_store(winsum + blockIdx.x, r);
 }
 
 // one CTA of COOP_THREADS threads per MSM
 __global__ void __launch_bounds__(COOP_THREADS) batch_final_kernel(const BatchDesc* d, const Xyzz* winsum,
                                                                     Jac* out) {
-    __shared__ Fq buf[8];
     const uint32_t i = blockIdx.x;
     const BatchDesc q = d[i];
-    const Jac j = coop_horner(buf, winsum + q.win_off, q.n ? (int)q.Wb : 0, (int)q.c);
+    const Jac j = coop_horner(winsum + q.win_off, q.n ? (int)q.Wb : 0, (int)q.c);
     if (threadIdx.x == 0) {
         st_elem<FqCfg>(&out[i].x, j.x);
         st_elem<FqCfg>(&out[i].y, j.y);

@@ -29,122 +29,127 @@ __device__ __forceinline__ void st_xyzz(Xyzz* p, const Xyzz& v) {
 }
 
 // ---------------------------------------------------------------------------
-// Final combination  sum_w 2^(c w) S_w  (Horner, (W - 1) c doublings).
+// Point arithmetic by quads of lanes, where the time is the latency of one
+// operation: the final combination  sum_w 2^(c w) S_w  (Horner, (W - 1) c
+// doublings), the trees of the bucket reduction and the merge of split buckets.
 //
-// It is one dependent chain, so its time is the latency of the products on
-// the chain.  One warp's Fq product is bound by the multiply pipe of its SM
-// sub-partition, so a thread cannot overlap two products; instead a CTA of
-// four warps (one per sub-partition) evaluates up to four independent products
-// of a formula at once: lane 0 of warp k computes product k, the results meet
-// in shared memory, and every thread keeps the whole point in registers and
-// does the additions itself.  A doubling (6M + 3S) becomes three product
-// levels, an addition (12M + 2S) four.
+// Lane k of a quad holds component k of a point (X, Y, ZZ, ZZZ) and computes
+// product k of the up to four independent products of a formula level; a
+// level's results reach the next one's operands by shuffles inside the quad.  An
+// addition takes four products of a warp, a doubling three, where one lane on
+// its own takes fourteen and nine, and a warp runs eight of them side by side.
+// All 32 lanes call these functions.  Coordinates lie in [0, 2p); ZZ of the
+// identity is zero itself, as are its other components.  Alone on a
+// sub-partition a quad addition takes 4400 clocks and a doubling 3250, a lane's
+// own addition 13100 and doubling 8700 (a product is 850-900 clocks of latency).
 
-static constexpr int COOP_THREADS = 128;
+static constexpr int COOP_THREADS = 32;
 
-struct Coop {
-    Fq* buf;  // shared, 2 x 4 elements (double-buffered result slots)
-    int par;
-};
+__device__ __forceinline__ int qd_lane() { return threadIdx.x & 3; }
 
-// r_k = a_k * b_k for k < cnt, all threads receive every result
-template <int CNT>
-__device__ __forceinline__ void coop_mul(Coop& co, const Fq& a0, const Fq& b0, const Fq& a1, const Fq& b1,
-                                         const Fq& a2, const Fq& b2, const Fq& a3, const Fq& b3, Fq& r0, Fq& r1,
-                                         Fq& r2, Fq& r3) {
-    const int wp = threadIdx.x >> 5;
-    Fq* slot = co.buf + 4 * co.par;
-    if ((threadIdx.x & 31) == 0 && wp < CNT) {
-        const Fq a = wp == 0 ? a0 : wp == 1 ? a1 : wp == 2 ? a2 : a3;
-        const Fq b = wp == 0 ? b0 : wp == 1 ? b1 : wp == 2 ? b2 : b3;
-        slot[wp] = fe_mul<FqCfg>(a, b);
-    }
-    __syncthreads();
-    r0 = slot[0];
-    if (CNT > 1) r1 = slot[1];
-    if (CNT > 2) r2 = slot[2];
-    if (CNT > 3) r3 = slot[3];
-    // the next call writes the other slot set; this one is rewritten only
-    // after every thread has passed the next barrier, i.e. read these results
-    co.par ^= 1;
+__device__ __forceinline__ Fq qd_shfl(const Fq& v, int src) {
+    Fq r;
+#pragma unroll
+    for (int j = 0; j < 8; j++) r.v[j] = __shfl_sync(0xffffffffu, v.v[j], src, 4);
+    return r;
 }
 
-// 2 * p, dbl-2008-s-1 in three product levels
-__device__ __forceinline__ Xyzz coop_dbl(Coop& co, const Xyzz& p) {
-    if (xyzz_is_id(p)) return p;
-    Fq d = fe_zero<FqCfg>();
-    const Fq u = fe_dbl<FqCfg>(p.y);
-    Fq v, xx;
-    coop_mul<2>(co, u, u, p.x, p.x, d, d, d, d, v, xx, d, d);
-    const Fq mm = fe_add<FqCfg>(fe_dbl<FqCfg>(xx), xx);
-    Fq w, s, m2, zz;
-    coop_mul<4>(co, u, v, p.x, v, mm, mm, v, p.zz, w, s, m2, zz);
+__device__ __forceinline__ Fq qd_xor2(const Fq& v) {
+    Fq r;
+#pragma unroll
+    for (int j = 0; j < 8; j++) r.v[j] = __shfl_xor_sync(0xffffffffu, v.v[j], 2);
+    return r;
+}
+
+__device__ __forceinline__ Fq qd_sel(bool c, const Fq& a, const Fq& b) {
+    Fq r;
+#pragma unroll
+    for (int j = 0; j < 8; j++) r.v[j] = c ? a.v[j] : b.v[j];
+    return r;
+}
+
+__device__ __forceinline__ Fq qd_load(const Xyzz* p) { return ld_elem<FqCfg>(reinterpret_cast<const Fq*>(p) + qd_lane()); }
+__device__ __forceinline__ void qd_store(Xyzz* p, const Fq& v) {
+    st_elem<FqCfg>(reinterpret_cast<Fq*>(p) + qd_lane(), fe_canon<FqCfg>(v));
+}
+
+// 2 p: dbl-2008-s-1 with (Y, 3/2 X^2) for (2 Y, 3 X^2), i.e. its result scaled
+// by (1/4, 1/8, 1/4, 1/8), the same point
+__device__ __forceinline__ Fq qd_dbl(const Fq& p) {
+    const int k = qd_lane();
+    // X^2, V = Y^2; M = 3/2 X^2
+    const Fq r = cmul_lazy(p, p);
+    Fq h = r;
+    limbs_half_mod<FqCfg>(h.v);
+    h = fe_add_lazy<FqCfg>(r, h);
+    const Fq V = qd_shfl(r, 1), M = qd_shfl(h, 0);
+    // S = X V, W = Y V, ZZ3 = ZZ V, M^2
+    const Fq r2 = cmul_lazy(qd_sel(k == 3, M, p), qd_sel(k == 3, M, V));
+    const Fq mm = qd_shfl(r2, 3), W = qd_shfl(r2, 1);
+    const Fq s2 = fe_add_lazy<FqCfg>(r2, r2);
+    const Fq x3 = fe_sub_lazy<FqCfg>(mm, s2);
+    const Fq t = fe_sub_lazy<FqCfg>(fe_add_lazy<FqCfg>(s2, r2), mm);  // S - X3
+    // M (S - X3), Y W, -, ZZZ W
+    const Fq r3 = cmul_lazy(qd_sel(k == 0, M, p), qd_sel(k == 0, t, W));
+    const Fq y3 = fe_sub_lazy<FqCfg>(qd_shfl(r3, 0), r3);
+    return qd_sel(k < 2, qd_sel(k == 0, x3, y3), qd_sel(k == 2, r2, r3));
+}
+
+// p + q (add-2008-s)
+__device__ __forceinline__ Fq qd_add(const Fq& p, const Fq& q) {
+    const int k = qd_lane();
+    const int zz = (threadIdx.x & 28) + 2;  // this quad's ZZ lane
+    const bool idp = (__ballot_sync(0xffffffffu, fe_is_zero<FqCfg>(p)) >> zz) & 1u;
+    const bool idq = (__ballot_sync(0xffffffffu, fe_is_zero<FqCfg>(q)) >> zz) & 1u;
+    // U1 = X1 ZZ2, S1 = Y1 ZZZ2, U2 = ZZ1 X2, S2 = ZZZ1 Y2
+    const Fq r = cmul_lazy(p, qd_xor2(q));
+    const Fq d = fe_sub_lazy<FqCfg>(qd_xor2(r), r);  // P = U2 - U1, R = S2 - S1 in lanes 0, 1
+    const unsigned zd = __ballot_sync(0xffffffffu, fe_is_zero<FqCfg>(fe_canon<FqCfg>(d))) >> (threadIdx.x & 28);
+    // P^2, R^2, ZZ1 ZZ2, ZZZ1 ZZZ2
+    const Fq r2 = cmul_lazy(qd_sel(k < 2, d, p), qd_sel(k < 2, d, q));
+    const Fq PP = qd_shfl(r2, 0), U1 = qd_shfl(r, 0);
+    // PPP = P PP, Q = U1 PP, ZZ3 = ZZ1 ZZ2 PP
+    const Fq r3 = cmul_lazy(qd_sel(k == 0, d, qd_sel(k == 1, U1, r2)), PP);
+    const Fq PPP = qd_shfl(r3, 0), S1 = qd_shfl(r, 1);
+    // lane 1 holds R^2 and Q
+    const Fq x3 = fe_sub_lazy<FqCfg>(fe_sub_lazy<FqCfg>(r2, PPP), fe_add_lazy<FqCfg>(r3, r3));
+    const Fq t = fe_sub_lazy<FqCfg>(r3, x3);
+    // S1 PPP, R (Q - X3), -, ZZZ3 = ZZZ1 ZZZ2 PPP
+    const Fq r4 = cmul_lazy(qd_sel(k == 0, S1, qd_sel(k == 1, d, r2)), qd_sel(k == 1, t, PPP));
+    const Fq y3 = fe_sub_lazy<FqCfg>(r4, qd_shfl(r4, 0));
+    Fq res = qd_sel(k < 2, qd_sel(k == 0, qd_shfl(x3, 1), y3), qd_sel(k == 2, r3, r4));
+    const bool same_x = (zd & 1u) && !idp && !idq;
+    if (__any_sync(0xffffffffu, same_x)) {
+        const Fq dd = qd_dbl(p);
+        if (same_x) res = qd_sel(zd & 2u, dd, fe_zero<FqCfg>());
+    }
+    return qd_sel(idq, p, qd_sel(idp, q, res));
+}
+
+// the point with canonical coordinates, in every lane
+__device__ __forceinline__ Xyzz qd_point(const Fq& p) {
     Xyzz r;
-    r.x = fe_sub<FqCfg>(fe_sub<FqCfg>(m2, s), s);
-    const Fq t = fe_sub<FqCfg>(s, r.x);
-    Fq zzz, wy, mt;
-    coop_mul<3>(co, w, p.zzz, w, p.y, mm, t, d, d, zzz, wy, mt, d);
-    r.y = fe_sub<FqCfg>(mt, wy);
-    r.zz = zz;
-    r.zzz = zzz;
-    return r;
+    r.x = qd_shfl(p, 0);
+    r.y = qd_shfl(p, 1);
+    r.zz = qd_shfl(p, 2);
+    r.zzz = qd_shfl(p, 3);
+    return xyzz_canon(r);
 }
 
-// p + q, add-2008-s in four product levels
-__device__ __forceinline__ Xyzz coop_add(Coop& co, const Xyzz& p, const Xyzz& q) {
-    if (xyzz_is_id(p)) return q;
-    if (xyzz_is_id(q)) return p;
-    Fq d = fe_zero<FqCfg>();
-    Fq u1, u2, s1, s2;
-    coop_mul<4>(co, p.x, q.zz, q.x, p.zz, p.y, q.zzz, q.y, p.zzz, u1, u2, s1, s2);
-    const Fq P = fe_sub<FqCfg>(u2, u1);
-    const Fq R = fe_sub<FqCfg>(s2, s1);
-    if (fe_is_zero<FqCfg>(P)) {
-        if (fe_is_zero<FqCfg>(R)) return coop_dbl(co, p);
-        return xyzz_identity();
-    }
-    Fq pp, zzp, zzzp, rr;
-    coop_mul<4>(co, P, P, p.zz, q.zz, p.zzz, q.zzz, R, R, pp, zzp, zzzp, rr);
-    Fq ppp, qq, zz;
-    coop_mul<3>(co, P, pp, u1, pp, zzp, pp, d, d, ppp, qq, zz, d);
-    Xyzz r;
-    r.x = fe_sub<FqCfg>(fe_sub<FqCfg>(fe_sub<FqCfg>(rr, ppp), qq), qq);
-    const Fq t = fe_sub<FqCfg>(qq, r.x);
-    Fq zzz, sp, rt;
-    coop_mul<3>(co, zzzp, ppp, s1, ppp, R, t, d, d, zzz, sp, rt, d);
-    r.y = fe_sub<FqCfg>(rt, sp);
-    r.zz = zz;
-    r.zzz = zzz;
-    return r;
-}
-
-// XYZZ -> Jacobian (X ZZ^2, Y ZZ^3, ZZZ); identity -> (0, 1, 0)
-__device__ __forceinline__ Jac coop_to_jac(Coop& co, const Xyzz& p) {
-    Jac r;
-    if (xyzz_is_id(p)) {
-        r.x = fe_zero<FqCfg>();
-        r.y = fe_one<FqCfg>();
-        r.z = fe_zero<FqCfg>();
-        return r;
-    }
-    Fq d = fe_zero<FqCfg>(), zz2, zz3;
-    coop_mul<1>(co, p.zz, p.zz, d, d, d, d, d, d, zz2, d, d, d);
-    coop_mul<2>(co, zz2, p.zz, p.x, zz2, d, d, d, d, zz3, r.x, d, d);
-    coop_mul<1>(co, p.y, zz3, d, d, d, d, d, d, r.y, d, d, d);
-    r.z = p.zzz;
-    return r;
-}
-
-// Horner over the W window sums win[0..W) of one MSM by the whole CTA
-// (COOP_THREADS threads); every thread returns the Jacobian result.
-__device__ __forceinline__ Jac coop_horner(Fq* sh_buf, const Xyzz* win, int W, int c) {
-    Coop co{sh_buf, 0};
-    Xyzz acc = W > 0 ? ld_xyzz(win + W - 1) : xyzz_identity();
+// Horner over the W window sums win[0..W) of one MSM by one warp (its quads
+// all compute the same)
+__device__ __forceinline__ Jac coop_horner(const Xyzz* win, int W, int c) {
+    Fq acc = fe_zero<FqCfg>();
+    if (W > 0) acc = qd_load(win + W - 1);
     for (int w = W - 2; w >= 0; w--) {
-        for (int i = 0; i < c; i++) acc = coop_dbl(co, acc);
-        acc = coop_add(co, acc, ld_xyzz(win + w));
+        const Fq next = qd_load(win + w);
+        // small scalars leave the top windows empty
+        const int dbl = __all_sync(0xffffffffu, fe_is_zero<FqCfg>(acc)) ? 0 : c;
+#pragma unroll 1
+        for (int i = 0; i < dbl; i++) acc = qd_dbl(acc);
+        acc = qd_add(acc, next);
     }
-    return coop_to_jac(co, acc);
+    return xyzz_to_jac(qd_point(acc));
 }
 
 // ---------------------------------------------------------------------------
@@ -160,9 +165,7 @@ __device__ __forceinline__ Jac coop_horner(Fq* sh_buf, const Xyzz* win, int W, i
 // is the right half's T.  So no thread multiplies its T by its segment's
 // number (about 1.5 log2 B additions' worth of doublings and additions each,
 // which was most of the reduction's work where segments are short), and what
-// is left is one short Horner chain a set.  Eight MSMs of 2^15 points (2^14
-// buckets each) reduce in 230 us against 700, one of 100003 points in 167
-// against 234 (ncu).
+// is left is one short Horner chain a set.
 //
 // Stages: (1) a block of RED_T threads sums RED_T segments and runs the tree
 // over each group of GS = min(G, RED_T) of them; (2) where a set has H = G / GS
@@ -175,21 +178,29 @@ static constexpr uint32_t RED_LG = 7;
 static constexpr uint32_t RED_MAX_G = RED_T * RED_T;
 static constexpr uint32_t RED_PLANES = RED_LG + 2;
 
-// Trees over the first 2^lg-leaf groups of Tp and Sp (either may be null),
-// RED_T leaves each; every thread of the block calls it after a barrier.  Node
-// base of level l holds T at Tp[base], V_k at Tp[base + 2^k] (k < l) and S at
-// Sp[base].
+// Trees over the groups of 2^lg leaves of Tp and Sp (either may be null), RED_T
+// leaves each, one addition a quad; every thread of the block calls it after a
+// barrier.  Node base of level l holds T at Tp[base], V_k at Tp[base + 2^k]
+// (k < l) and S at Sp[base].
 __device__ __forceinline__ void red_tree(Xyzz* Tp, Xyzz* Sp, uint32_t lg) {
+    const uint32_t quad = threadIdx.x >> 2;
+#pragma unroll 1
     for (uint32_t l = 1; l <= lg; l++) {
-        // one addition a thread: at most RED_T of them on every level
-        const uint32_t nodes = RED_T >> l, base = (threadIdx.x & (nodes - 1)) << l;
-        const uint32_t r = threadIdx.x >> (RED_LG - l);
-        Xyzz* dst = nullptr;
-        if (r == 0)
-            dst = Sp ? Sp + base : nullptr;
-        else if (r <= l)
-            dst = Tp ? Tp + base + (r >= 2 ? 1u << (r - 2) : 0u) : nullptr;
-        if (dst) *dst = xyzz_add(*dst, dst[1u << (l - 1)]);
+        // additions: row r of the level's nodes; row 0 is S, row 1 T, row 2 + k V_k
+        const uint32_t nodes = RED_T >> l, first = Sp ? 0u : nodes, last = Tp ? nodes * (l + 1) : nodes;
+#pragma unroll 1
+        for (uint32_t a0 = first; a0 < last; a0 += RED_T / 4) {
+            const uint32_t a = a0 + quad, r = a >> (RED_LG - l), base = (a & (nodes - 1)) << l;
+            Xyzz* dst = r == 0 ? Sp + base : Tp + base + (r >= 2 ? 1u << (r - 2) : 0u);
+            const bool live = a < last;
+            Fq p = fe_zero<FqCfg>(), q = p;
+            if (live) {
+                p = reinterpret_cast<const Fq*>(dst)[qd_lane()];
+                q = reinterpret_cast<const Fq*>(dst + (1u << (l - 1)))[qd_lane()];
+            }
+            p = qd_add(p, q);
+            if (live) reinterpret_cast<Fq*>(dst)[qd_lane()] = p;
+        }
         __syncthreads();
     }
 }
@@ -220,7 +231,7 @@ __device__ __forceinline__ void red_groups(Xyzz* Tp, Xyzz* Sp, const Xyzz& S, co
     const uint32_t planes = lg + 1 + (H > 1 ? 1u : 0u);
     if (live && p < planes) {
         const Xyzz v = p == 0 ? Sp[base] : Tp[base + (p <= lg ? 1u << (p - 1) : 0u)];
-        st_xyzz(out + p * H + h, v);
+        st_xyzz(out + p * H + h, xyzz_canon(v));
     }
 }
 
@@ -233,24 +244,29 @@ __device__ __forceinline__ void red_plane(Xyzz* sm, Xyzz* set, uint32_t H, uint3
     red_tree(t_plane ? sm : nullptr, t_plane ? nullptr : sm, lg);
     Xyzz* out = set + RED_PLANES * H;
     if (!t_plane) {
-        if (i == 0) st_xyzz(out + p, sm[0]);
+        if (i == 0) st_xyzz(out + p, xyzz_canon(sm[0]));
     } else if (i < lg) {
-        st_xyzz(out + p + i, sm[1u << i]);
+        st_xyzz(out + p + i, xyzz_canon(sm[1u << i]));
     }
 }
 
-// stage 3 by COOP_THREADS threads: the set's sum
-__device__ __forceinline__ Xyzz red_horner(Fq* sh_buf, const Xyzz* set, uint32_t G, uint32_t seg) {
+// stage 3 by one warp: the set's sum, component qd_lane() in every quad
+__device__ __forceinline__ Fq red_horner(const Xyzz* set, uint32_t G, uint32_t seg) {
     const uint32_t H = G > RED_T ? G / RED_T : 1u;
     const Xyzz* v = H > 1 ? set + RED_PLANES * H : set;
-    Coop co{sh_buf, 0};
-    Xyzz acc = xyzz_identity();
-    for (uint32_t k = 31u - (uint32_t)__clz((int)G); k > 0; k--) {
-        acc = coop_dbl(co, acc);
-        acc = coop_add(co, acc, ld_xyzz(v + k));
+    Fq acc = fe_zero<FqCfg>();
+    // the bits of the segment number from the top, seg's doublings, then S
+    uint32_t k = 31u - (uint32_t)__clz((int)G), s = seg;
+#pragma unroll 1
+    while (s) {
+        if (k > 0 || s > 1) acc = qd_dbl(acc);
+        if (k > 0 || s == 1) acc = qd_add(acc, qd_load(v + k));
+        if (k > 0)
+            k--;
+        else
+            s >>= 1;
     }
-    for (uint32_t s = seg; s > 1; s >>= 1) acc = coop_dbl(co, acc);
-    return coop_add(co, acc, ld_xyzz(v));
+    return acc;
 }
 
 }  // namespace zk
