@@ -35,6 +35,19 @@ def test_batch_inverse(O, gpu, n, with_scratch):
     assert (H.to_host(d) == O.batch_inv(a)).all()
 
 
+# around the sizes where a thread takes 2, 4 and 8 elements
+@pytest.mark.parametrize("n", [511, 512, 513, 151552, 151553, 303104, 303105])
+def test_batch_inverse_elements_per_thread(O, gpu, n):
+    H = gpu.host
+    a = O.rand_fr(n, 300 + n % 997)
+    a[n // 2] = 0
+    a[n - 1] = 0
+    out = H.empty_fr(n)
+    H.batch_inverse(out, H.to_device(a))
+    torch.cuda.synchronize()
+    assert (H.to_host(out) == O.batch_inv(a)).all()
+
+
 # 2049 and 4097: a last tile of one element; (1 << 22) + 3: 2049 tiles, so the
 # look-back windows of 32 tiles wrap many times
 @pytest.mark.parametrize("n", [1, 7, 2048, 2049, 4097, 300000, 1 << 22, (1 << 22) + 3])

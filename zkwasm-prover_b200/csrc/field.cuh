@@ -590,20 +590,6 @@ ZK_HD Fe<C> fe_pow_u32(Fe<C> a, uint32_t e) {
     return r;
 }
 
-// a^(m-2): multiplicative inverse by Fermat's little theorem (0 maps to 0).
-// 8-limb helpers of the binary inversion
-ZK_HD bool limbs_is_one(const uint32_t x[8]) {
-    uint32_t o = x[0] ^ 1u;
-#pragma unroll
-    for (int j = 1; j < 8; j++) o |= x[j];
-    return o == 0;
-}
-
-ZK_HD bool limbs_geq(const uint32_t a[8], const uint32_t b[8]) {
-    uint32_t t[8];
-    return sub8_borrow(t, a, b) == 0;
-}
-
 ZK_HD void limbs_shr1(uint32_t x[8]) {
 #pragma unroll
     for (int j = 0; j < 7; j++) x[j] = (x[j] >> 1) | (x[j + 1] << 31);
@@ -622,64 +608,161 @@ ZK_HD void limbs_half_mod(uint32_t x[8]) {
     limbs_shr1(x);
 }
 
-// x - y mod m for x, y < m
-template <class C>
-ZK_HD void limbs_sub_mod(uint32_t x[8], const uint32_t y[8]) {
-    uint32_t t[8], u[8], m[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) m[j] = C::M(j);
-    const uint32_t br = sub8_borrow(t, x, y);
-    add8_carry(u, t, m);
-    select8(x, br, u, t);
+// ---------------------------------------------------------------------------
+// Inverse by division steps (D. J. Bernstein and B.-Y. Yang, "Fast
+// constant-time gcd computation and modular inversion", 2019), in the variant
+// that starts at delta = 1/2.  A step takes (delta, f, g), f odd, to
+//     (1 - delta, g, (g - f) / 2)              if delta > 0 and g is odd,
+//     (1 + delta, f, (g + (g mod 2) f) / 2)    otherwise,
+// and from f = m, g = a it reaches g = 0, f = +-1.  Thirty steps look at the
+// lowest 30 bits of f and g only, so they run on two words and are collected in
+// a matrix of 31-bit entries that is then applied to the long f, g and to the
+// cofactors d, e (f = d a, g = e a mod m, each application an exact division by
+// 2^30 after adding the multiple of m that makes it one).  At most 590 steps
+// for 256-bit m; the loop ends when g is zero.
+//
+// Numbers are nine limbs of 30 bits, the top one signed.  Against the binary
+// Euclid it replaces, one bit of 8-limb chains at a time, a step is a few
+// 32-bit operations: 39500 clocks (20 us) for one thread against about 70000.
+
+struct Inv30 {
+    int32_t v[9];
+};
+
+struct InvMat {
+    int32_t u, v, q, r;
+};
+
+// 30 division steps from the low words of f and g; twice delta in and out
+ZK_HD InvMat inv_steps(int32_t& delta2, uint32_t f, uint32_t g) {
+    uint32_t u = 1, v = 0, q = 0, r = 1;
+#pragma unroll 6
+    for (int i = 0; i < 30; i++) {
+        const bool odd = g & 1u;
+        const bool swap = odd && delta2 > 0;
+        // (f, g) <- (g, -f) with its matrix rows, then g += f
+        const uint32_t f0 = f, u0 = u, v0 = v;
+        f = swap ? g : f;
+        u = swap ? q : u;
+        v = swap ? r : v;
+        g = swap ? 0u - f0 : g;
+        q = swap ? 0u - u0 : q;
+        r = swap ? 0u - v0 : r;
+        delta2 = swap ? 2 - delta2 : delta2 + 2;
+        g += odd ? f : 0u;
+        q += odd ? u : 0u;
+        r += odd ? v : 0u;
+        g = (uint32_t)((int32_t)g >> 1);
+        u <<= 1;
+        v <<= 1;
+    }
+    return {(int32_t)u, (int32_t)v, (int32_t)q, (int32_t)r};
 }
 
-// Inverse of a Montgomery-form element (zero maps to zero).  Binary extended
-// Euclid (variable time) on the representative A = a R: u, v start at A and
-// m with u = x1 A, v = x2 A (mod m) kept invariant; halving and subtracting
-// until u or v is 1 gives A^-1, and the Montgomery product with R^3 turns it
-// into a^-1 R.  Each step is a few short 8-limb chains, so one thread takes
-// a fraction of the latency of the ~380 dependent products of a^(m-2).
+// a <- (x a + y b + k m) / 2^30 with k the multiple of m that clears the low
+// limb (MOD), or 0 where it is clear already
+template <class C, bool MOD>
+ZK_HD Inv30 inv_row(const Inv30& a, const Inv30& b, int32_t x, int32_t y, const int32_t m[9], uint32_t minv) {
+    const int64_t M30 = (1 << 30) - 1;
+    int64_t c = (int64_t)x * a.v[0] + (int64_t)y * b.v[0];
+    int32_t k = 0;
+    if (MOD) {
+        k = (int32_t)(((uint32_t)c * minv) & (uint32_t)M30);  // minv = -m^-1 mod 2^30
+        c += (int64_t)k * m[0];
+    }
+    c >>= 30;
+    Inv30 r;
+#pragma unroll
+    for (int i = 1; i < 9; i++) {
+        c += (int64_t)x * a.v[i] + (int64_t)y * b.v[i];
+        if (MOD) c += (int64_t)k * m[i];
+        r.v[i - 1] = (int32_t)(c & M30);
+        c >>= 30;
+    }
+    r.v[8] = (int32_t)c;
+    return r;
+}
+
+// limb i of nine 30-bit limbs of an 8-word number
+ZK_HD int32_t inv_limb(const uint32_t x[8], int i) {
+    const int b = 30 * i, w = b >> 5, o = b & 31;
+    uint32_t t = x[w] >> o;
+    if (o > 2 && w + 1 < 8) t |= x[w + 1] << (32 - o);
+    return (int32_t)(t & 0x3fffffffu);
+}
+
+// Inverse of a Montgomery-form element (zero maps to zero): the inverse of the
+// representative A = a R, then the Montgomery product with R^3 gives a^-1 R.
 template <class C>
 ZK_HD Fe<C> fe_inv(const Fe<C>& a) {
     if (fe_is_zero<C>(a)) return a;
-    uint32_t u[8], v[8], x1[8], x2[8];
+    uint32_t mw[8];
+    int32_t m[9];
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-        u[j] = a.v[j];
-        v[j] = C::M(j);
-        x1[j] = j == 0 ? 1u : 0u;
-        x2[j] = 0u;
-    }
-    bool first = true;
-    for (;;) {
-        while (!(u[0] & 1u)) {
-            limbs_shr1(u);
-            limbs_half_mod<C>(x1);
-        }
-        while (!(v[0] & 1u)) {
-            limbs_shr1(v);
-            limbs_half_mod<C>(x2);
-        }
-        if (limbs_is_one(u)) break;
-        if (limbs_is_one(v)) {
-            first = false;
-            break;
-        }
-        if (limbs_geq(u, v)) {
-            sub8_borrow(u, u, v);
-            limbs_sub_mod<C>(x1, x2);
-        } else {
-            sub8_borrow(v, v, u);
-            limbs_sub_mod<C>(x2, x1);
-        }
-    }
-    Fe<C> x, r3;
+    for (int j = 0; j < 8; j++) mw[j] = C::M(j);
+    Inv30 f, g, d, e;
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-        x.v[j] = first ? x1[j] : x2[j];
-        r3.v[j] = C::R3(j);
+    for (int i = 0; i < 9; i++) {
+        m[i] = inv_limb(mw, i);
+        f.v[i] = m[i];
+        g.v[i] = inv_limb(a.v, i);
+        d.v[i] = 0;
+        e.v[i] = i == 0;
     }
-    return fe_mul<C>(x, r3);
+    int32_t delta2 = 1;
+    // d and e gain at most m a round: they stay inside (-21 m, 21 m)
+    for (int round = 0; round < 20; round++) {
+        const InvMat t = inv_steps(delta2, (uint32_t)f.v[0] | ((uint32_t)f.v[1] << 30),
+                                   (uint32_t)g.v[0] | ((uint32_t)g.v[1] << 30));
+        const Inv30 nd = inv_row<C, true>(d, e, t.u, t.v, m, C::INV);
+        e = inv_row<C, true>(d, e, t.q, t.r, m, C::INV);
+        d = nd;
+        const Inv30 nf = inv_row<C, false>(f, g, t.u, t.v, m, 0);
+        g = inv_row<C, false>(f, g, t.q, t.r, m, 0);
+        f = nf;
+        int32_t nz = 0;
+#pragma unroll
+        for (int i = 0; i < 9; i++) nz |= g.v[i];
+        if (!nz) break;
+    }
+    // f = +-1 and f = d A: the inverse is f d.  Into [0, m): add 32 m, then take
+    // off 32 m, 16 m, ..., m where that leaves it non-negative
+    const int32_t sign = f.v[8] < 0 ? -1 : 1;
+    int32_t x[9];
+    {
+        int64_t c = 0;
+#pragma unroll
+        for (int i = 0; i < 9; i++) {
+            c += (int64_t)sign * d.v[i] + ((int64_t)m[i] << 5);
+            x[i] = i < 8 ? (int32_t)(c & 0x3fffffff) : (int32_t)c;
+            c >>= 30;
+        }
+    }
+#pragma unroll 1
+    for (int s = 5; s >= 0; s--) {
+        int32_t y[9];
+        int64_t c = 0;
+#pragma unroll
+        for (int i = 0; i < 9; i++) {
+            c += (int64_t)x[i] - ((int64_t)m[i] << s);
+            y[i] = i < 8 ? (int32_t)(c & 0x3fffffff) : (int32_t)c;
+            c >>= 30;
+        }
+        const bool neg = y[8] < 0;
+#pragma unroll
+        for (int i = 0; i < 9; i++) x[i] = neg ? x[i] : y[i];
+    }
+    Fe<C> r, r3;
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+        const int b = 32 * w, k = b / 30, o = b % 30;
+        uint32_t t = (uint32_t)x[k] >> o;
+        t |= (uint32_t)x[k + 1] << (30 - o);
+        if (60 - o < 32 && k + 2 < 9) t |= (uint32_t)x[k + 2] << (60 - o);
+        r.v[w] = t;
+        r3.v[w] = C::R3(w);
+    }
+    return fe_mul<C>(r, r3);
 }
 
 // n-bit field of a canonical (non-Montgomery) 256-bit value starting at bit `start`

@@ -63,13 +63,14 @@ __device__ Fr block_excl_scan_fr(int op, const Fr& v, Fr* wsm, Fr& total) {
 }
 
 // ------------------------------------------------------------ batch inverse
-// Montgomery's trick over a block of ST * SK elements: one field inversion per
-// block.  Thread t owns elements base + t + ST*k (coalesced); its chunk
-// product is combined with the exclusive prefix E_t and suffix S_t of the
-// other threads' products, so inv(chunk_t) = inv(total) * S_t * E_t, and the
-// chunk is unwound locally.  The element value comes from a functor that is
-// evaluated twice (forward and backward) instead of being stored, so the
-// kernel needs no scratch memory.  Zero elements invert to zero.
+// Montgomery's trick over a block of ST * K elements: one field inversion per
+// block.  Thread t owns elements base + t + ST*k (coalesced); a binary tree in
+// shared memory multiplies the threads' chunk products up to the block's,
+// whose inverse goes down again (a node's inverse times its sibling's product
+// is its child's), and each chunk is unwound locally.  The element value comes
+// from a functor that is evaluated twice (forward and backward) instead of
+// being stored, so the kernel needs no scratch memory.  Zero elements invert
+// to zero.
 
 struct SrcPlus {  // in[i] + c  (c optional)
     const Fr* in;
@@ -130,51 +131,83 @@ __global__ void __launch_bounds__(ST) batch_prod_kernel(Src src, uint32_t n, Fr*
 }
 
 // inv_tots: the inverses of the block products (three-phase form), or null
-// to invert each block's product in the block (one Fermat inversion per block)
-// The per-thread prefix products live in shared memory (SK x ST elements,
-// 64 KB), not registers: at about 80 registers three blocks fit an SM, so
-// while one block waits on its inversion (about 36 us on one thread) two
-// others compute.
-static constexpr size_t BATCH_INV_SMEM = (size_t)SK * ST * sizeof(Fr);
+// to invert each block's product in the block.
+// The per-thread prefix products live in shared memory (K x ST elements, the
+// last plane holding the tree's leaves, and ST inner nodes), not registers: at
+// K = 8 three blocks fit an SM.  The tree takes 36 products of whole warps a
+// block, where exclusive prefixes and suffixes of the chunk products by two
+// block scans took 176.  Bound by the chain of tree and inversion while it
+// waits (2^15 elements: 114 -> 41 us with K = 2; 2^20: 218 -> 157 us).
+template <int K>
+static constexpr size_t batch_inv_smem() {
+    return (size_t)(K + 1) * ST * sizeof(Fr);
+}
 
-template <class Src, class Dst>
+template <int K, class Src, class Dst>
 __global__ void __launch_bounds__(ST, 3) batch_inv_kernel(Src src, Dst dst, uint32_t n, const Fr* inv_tots) {
-    __shared__ Fr wsm[32];
-    __shared__ Fr rev[ST];
-    __shared__ Fr inv_tot;
     extern __shared__ uint4 smem_u4[];
     Fr* pre_sm = reinterpret_cast<Fr*>(smem_u4);  // [k][t]
-    const size_t base = (size_t)blockIdx.x * SBLK;
+    Fr* leaf = pre_sm + (K - 1) * ST;             // heap nodes ST + t
+    Fr* node = pre_sm + K * ST;                   // heap nodes 1 .. ST - 1
+    const size_t base = (size_t)blockIdx.x * (ST * K);
     const int t = threadIdx.x;
     const Fr one = fe_one<FrCfg>();
     Fr run = one;
 #pragma unroll
-    for (int k = 0; k < SK; k++) {
+    for (int k = 0; k < K; k++) {
         const size_t i = base + t + (size_t)ST * k;
         Fr a = one;
         if (i < n) {
             a = src((uint32_t)i);
             if (fe_is_zero<FrCfg>(a)) a = one;
         }
-        run = fe_mul<FrCfg>(run, a);
+        run = k ? fe_mul<FrCfg>(run, a) : a;
         pre_sm[k * ST + t] = run;
     }
-    Fr tot;
-    Fr E = block_excl_scan_fr(OP_MUL, run, wsm, tot);
-    rev[ST - 1 - t] = run;
     __syncthreads();
-    Fr rv = rev[t];
+    // up: node i = node 2i * node 2i + 1; the nodes below 64 are warp 0's
+#pragma unroll 1
+    for (int h = ST / 2; h >= 32; h >>= 1) {
+        if (t < h) {
+            const Fr* c = h == ST / 2 ? leaf + 2 * t : node + 2 * (h + t);
+            node[h + t] = fe_mul<FrCfg>(c[0], c[1]);
+        }
+        __syncthreads();
+    }
+    if (t < 32) {
+#pragma unroll 1
+        for (int h = 16; h >= 1; h >>= 1) {
+            if (t < h) node[h + t] = fe_mul<FrCfg>(node[2 * (h + t)], node[2 * (h + t) + 1]);
+            __syncwarp();
+        }
+        if (t == 0) node[1] = inv_tots ? ld_elem<FrCfg>(inv_tots + blockIdx.x) : fe_inv<FrCfg>(node[1]);
+        __syncwarp();
+        // down: the inverses of a node's children
+#pragma unroll 1
+        for (int h = 1; h <= 16; h <<= 1) {
+            if (t < h) {
+                Fr* c = node + 2 * (h + t);
+                const Fr inv = node[h + t], l = c[0], r = c[1];
+                c[0] = fe_mul<FrCfg>(inv, r);
+                c[1] = fe_mul<FrCfg>(inv, l);
+            }
+            __syncwarp();
+        }
+    }
     __syncthreads();
-    Fr tot2;
-    Fr Srev = block_excl_scan_fr(OP_MUL, rv, wsm, tot2);
-    rev[ST - 1 - t] = Srev;
-    __syncthreads();
-    Fr S = rev[t];
-    if (t == 0) inv_tot = inv_tots ? ld_elem<FrCfg>(inv_tots + blockIdx.x) : fe_inv<FrCfg>(tot);
-    __syncthreads();
-    Fr cur = fe_mul<FrCfg>(fe_mul<FrCfg>(inv_tot, S), E);
+#pragma unroll 1
+    for (int h = 32; h < ST; h <<= 1) {
+        if (t < h) {
+            Fr* c = h == ST / 2 ? leaf + 2 * t : node + 2 * (h + t);
+            const Fr inv = node[h + t], l = c[0], r = c[1];
+            c[0] = fe_mul<FrCfg>(inv, r);
+            c[1] = fe_mul<FrCfg>(inv, l);
+        }
+        __syncthreads();
+    }
+    Fr cur = leaf[t];
 #pragma unroll
-    for (int k = SK - 1; k >= 0; k--) {
+    for (int k = K - 1; k >= 0; k--) {
         const size_t i = base + t + (size_t)ST * k;
         Fr a = one;
         bool zero = true;
@@ -183,8 +216,11 @@ __global__ void __launch_bounds__(ST, 3) batch_inv_kernel(Src src, Dst dst, uint
             zero = fe_is_zero<FrCfg>(a);
             if (zero) a = one;
         }
-        Fr inv_k = k ? fe_mul<FrCfg>(cur, pre_sm[(k - 1) * ST + t]) : cur;
-        cur = fe_mul<FrCfg>(cur, a);
+        Fr inv_k = cur;
+        if (k) {
+            inv_k = fe_mul<FrCfg>(cur, pre_sm[(k - 1) * ST + t]);
+            cur = fe_mul<FrCfg>(cur, a);
+        }
         if (i < n) dst((uint32_t)i, zero ? fe_zero<FrCfg>() : inv_k);
     }
 }
@@ -199,31 +235,38 @@ size_t batch_inv_scratch_elems(uint32_t n) {
 // With scratch of batch_inv_scratch_elems(n) and n above 2^22: (1) block
 // products, (2) their inverses by the same routine (recursively, one field
 // inversion at the top), (3) every block unwound with its product's inverse.
-// Otherwise each block inverts its own product (binary extended Euclid, about
-// 30 us of one thread while the block waits): measured on B200 this is the
-// faster form up to 2^22 elements (0.078 against 0.136 ms at 2^16, 0.57
-// against 0.64 ms at 2^22), the extra pass of the three-phase form costing
-// more than the inversion stalls that other resident blocks partly hide.
+// Otherwise each block inverts its own product: the extra pass of
+// the three-phase form costs more than the inversions that other resident
+// blocks partly hide (measured before the division steps at 2^16 and 2^22).
 static constexpr uint32_t BATCH_INV_THREE_PHASE_ABOVE = 1u << 22;
+
+template <int K, class Src, class Dst>
+static cudaError_t launch_batch_inv_k(Src src, Dst dst, uint32_t n, const Fr* inv_tots, cudaStream_t s) {
+    static SmemOptIn opt;
+    ZK_CHECK(opt.ensure(batch_inv_kernel<K, Src, Dst>, (int)batch_inv_smem<K>()));
+    batch_inv_kernel<K, Src, Dst><<<(n + ST * K - 1) / (ST * K), ST, batch_inv_smem<K>(), s>>>(src, dst, n, inv_tots);
+    return cudaGetLastError();
+}
 
 template <class Src, class Dst>
 static cudaError_t launch_batch_inv(Src src, Dst dst, uint32_t n, Fr* scratch, size_t scratch_elems, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    static SmemOptIn opt;
-    ZK_CHECK(opt.ensure(batch_inv_kernel<Src, Dst>, (int)BATCH_INV_SMEM));
-    const uint32_t nb = (n + SBLK - 1) / SBLK;
     if (n > BATCH_INV_THREE_PHASE_ABOVE && scratch && scratch_elems >= batch_inv_scratch_elems(n)) {
+        const uint32_t nb = (n + SBLK - 1) / SBLK;
         Fr* tot = scratch;
         Fr* inv = scratch + nb;
         batch_prod_kernel<Src><<<nb, ST, 0, s>>>(src, n, tot);
         ZK_CHECK(cudaGetLastError());
         ZK_CHECK(launch_batch_inv(SrcPlus{tot, nullptr}, DstStore{inv, 0}, nb, scratch + 2 * (size_t)nb,
                                   scratch_elems - 2 * (size_t)nb, s));
-        batch_inv_kernel<Src, Dst><<<nb, ST, BATCH_INV_SMEM, s>>>(src, dst, n, inv);
-        return cudaGetLastError();
+        return launch_batch_inv_k<SK>(src, dst, n, inv, s);
     }
-    batch_inv_kernel<Src, Dst><<<nb, ST, BATCH_INV_SMEM, s>>>(src, dst, n, nullptr);
-    return cudaGetLastError();
+    // elements a thread: eight once that fills the SMs twice over, fewer below,
+    // where a block's chain of dependent products is the time (2^15 elements:
+    // 16 blocks at eight, 64 at two)
+    if (n > 4 * 2 * 148 * ST) return launch_batch_inv_k<8>(src, dst, n, nullptr, s);
+    if (n > 2 * 2 * 148 * ST) return launch_batch_inv_k<4>(src, dst, n, nullptr, s);
+    return launch_batch_inv_k<2>(src, dst, n, nullptr, s);
 }
 
 cudaError_t batch_inverse(Fr* out, const Fr* in, const Fr* c, uint32_t n, int accumulate, Fr* scratch,
