@@ -109,6 +109,35 @@ def test_cosets_and_combine(O, gpu, P, ext_bits, pairs):
     assert (_h(out) == exp).all()
 
 
+# two passes with every remainder of the in-block radix (7+6, 6+8, 9+9, 11+10)
+# and three (11+6+6): the coset's factors come from the first pass's own table
+@pytest.mark.parametrize("log_n", [13, 14, 16, 18, 21, 23])
+@pytest.mark.parametrize("pairs", [False, True])
+def test_coset_transform_of_several_passes(O, gpu, P, log_n, pairs):
+    L = gpu.load_library()
+    n, cols, stride = 1 << log_n, 2, (1 << log_n) + 24
+    tab = P.Tables(log_n)
+    w2 = O.omega(log_n + 1)
+    shift = RC.ZETA * w2 % O.R_MOD
+    twist = P.powers(1, shift, n)
+    tw = tab.tw
+    if pairs:
+        tw, tp = (torch.empty((2 * n, 4), dtype=torch.int64, device="cuda") for _ in range(2))
+        assert L.zkp_shoup_pairs(tw.data_ptr(), tab.tw.data_ptr(), n, 0) == 0
+        assert L.zkp_shoup_pairs(tp.data_ptr(), twist.data_ptr(), n, 0) == 0
+        twist = tp
+    coeff = O.rand_fr(cols * stride, 190 + log_n)
+    src = RC.Dev().put(coeff)
+    tmp = torch.empty((cols * n, 4), dtype=torch.int64, device="cuda")
+    out = torch.empty((cols * stride, 4), dtype=torch.int64, device="cuda")
+    assert L.zkp_ntt_batch_twisted(out.data_ptr(), src.data_ptr(), tmp.data_ptr(), tw.data_ptr(), twist.data_ptr(), 0,
+                                   log_n, cols, stride, stride, int(pairs), 0) == 0
+    got = _h(out)
+    for c in range(cols if log_n < 20 else 1):
+        exp = O.coset_ntt(coeff[c * stride:c * stride + n], log_n, log_n + 1, RC.ZETA)[1::2]
+        assert (got[c * stride:c * stride + n] == exp).all(), c
+
+
 def test_eval_h_fused_matches_restatement(O, gpu, P):
     """Every family of zkp_eval_h_fused on random columns (rotation scale 2,
     as on a whole extended domain of E = 2) against the oracle's restatement of

@@ -625,6 +625,11 @@ static cudaError_t extend_impl(void* ext_out, void* coeff_out, const void* lagra
         f.coeff_ys = n;
         f.sub_ys = n * E;
         f.pairs = pairs;
+        // ext_out is written by the last pass only: until then its head holds
+        // the cosets' sub-stage factors (2 R entries a coset, n >= 64 R)
+        f.ctab = F(ext_out);
+        ZK_CHECK(zk::ntt_coset_table(F(ext_out), f.stab, (size_t)1 << rad[1], log_n - rad[1], tw, log_n, rad[1], (int)E,
+                                     pairs, stream));
         ZK_CHECK(ntt_fused_extend(f, rad[1], ncols, stream));
         ZK_MARK(3);
         // 3. last pass of each coset's forward transform, interleaved output

@@ -23,6 +23,7 @@ struct NttPassArgs {
     size_t src_zs, dst_zs;  // per-sub-transform strides (blockIdx.z), elements
     size_t in_mul_zs;
     int pairs;           // tw, in_mul and scale hold (w, w') pairs (two elements an entry)
+    const Fr* ctab;      // first pass of a coset transform: its factors (ntt_coset_table), with in_mul
 };
 
 cudaError_t ntt_pass(const NttPassArgs& a, int log_r, unsigned ny, unsigned nz, cudaStream_t s);
@@ -37,10 +38,15 @@ struct FusedExtendArgs {
     const Fr* tw;      // w^i, n entries
     const Fr* wtab;    // E * n
     const Fr* stab;    // E * 2^log_r
+    const Fr* ctab;    // E * 2^(log_r + 1) entries (ntt_coset_table from stab)
     int log_n, E;
     size_t src_ys, coeff_ys, sub_ys;
     int pairs;         // every table holds (w, w') pairs (two elements an entry)
 };
+// sub-stage factors of a coset transform's first pass, 2^(log_r + 1) entries a
+// coset, from the powers of its shift (see ntt.cu)
+cudaError_t ntt_coset_table(Fr* ctab, const Fr* pw, size_t pw_zs, int pw_shift, const Fr* tw, int log_n, int log_r,
+                            int cosets, int pairs, cudaStream_t s);
 cudaError_t ntt_fused_extend(const FusedExtendArgs& a, int log_r, unsigned ncols, cudaStream_t s);
 cudaError_t ntt_fused_tables(Fr* wtab, Fr* stab, const Fr* tw, const Fr* shift, const Fr* w_ext, int log_n, int log_r,
                              int ext_bits, cudaStream_t s, bool pairs = false);

@@ -5,11 +5,20 @@
 // P_t = R_1 * ... * R_{t-1}.  Work item q in [0, n/R_t) with J = q mod P_t and
 // Q = q / P_t:
 //     reads   x[q + (n/R_t) * i]                       i < R_t
-//     y_j   = sum_i x_i w_{R_t}^{ij}                   (in shared memory)
-//     writes  dst[J + P_t*j + P_t*R_t*Q] = y_j * w_n^{P_t*Q*j}
+//     y_j   = sum_i x_i w_{P_t R_t}^{J i} w_{R_t}^{ij}  (in shared memory)
+//     writes  dst[J + P_t*j + P_t*R_t*Q] = y_j
 // so the final pass leaves X[j] = sum_i x_i w_n^{ij} in natural order.  Inside a
 // CTA the radix-R_t DFT is itself a Stockham sequence of radix-8 (then 4 or 2)
-// sub-stages held in registers, exchanging through shared memory.
+// sub-stages held in registers, exchanging through shared memory, each of the
+// same form with P_s = 8^s: input i of an item is multiplied by
+// w_{P R}^{J i} over the indexes of pass and sub-stage together, then a DFT of
+// eight follows.  Twiddles come before the DFT (decimation in time), so that
+//   - the first sub-stage of the first pass has none;
+//   - a factor common to all inputs (the scale n^-1) costs one product per
+//     eight elements: it goes into the eight factors of an item's first
+//     sub-stage, where input 0 otherwise has none;
+//   - a coset shift s (X[j] = sum_k x_k s^k w^{jk}) only changes factors that
+//     are multiplied by anyway: see ntt_coset_table_kernel.
 //
 // Twiddles come from the natural table w^i (i < n) that expand_omega_buffer
 // builds; a sub-stage twiddle w_R^e is entry e * (n/R).
@@ -94,6 +103,12 @@ struct TwM {
         return nt_mulz3(v0, k0.w, v1, k1.w, v2, k2.w);
     }
     static __host__ __device__ __forceinline__ const Fr* off(const Fr* t, size_t i) { return t + i; }
+    static constexpr int EW = 1;  // elements an entry
+    // the entry's value (in this layout's form) and the entry of a value
+    static __device__ __forceinline__ K of(const Fr& v) { return {v}; }
+    static __device__ __forceinline__ K prod(const K& a, const K& b) { return {nt_mul(a.w, b.w)}; }
+    static __device__ __forceinline__ K sm(const Fr* t) { return {t[0]}; }
+    static __device__ __forceinline__ void put(Fr* t, const K& k) { t[0] = k.w; }
 };
 struct TwS {
     struct K {
@@ -111,12 +126,22 @@ struct TwS {
         return nt_shoup3(v0, k0.w, k0.wp, v1, k1.w, k1.wp, v2, k2.w, k2.wp);
     }
     static __host__ __device__ __forceinline__ const Fr* off(const Fr* t, size_t i) { return t + 2 * i; }
+    static constexpr int EW = 2;
+    static __device__ __forceinline__ K of(const Fr& v) {
+        return {v, fe_shoup_companion<FrCfg>(fe_to_mont<FrCfg>(v))};
+    }
+    static __device__ __forceinline__ K prod(const K& a, const K& b) {
+        return of(fe_canon<FrCfg>(nt_shoup(a.w, b.w, b.wp)));
+    }
+    static __device__ __forceinline__ K sm(const Fr* t) { return {t[0], t[1]}; }
+    static __device__ __forceinline__ void put(Fr* t, const K& k) {
+        t[0] = k.w;
+        t[1] = k.wp;
+    }
 };
 
 
 // ---------------------------------------------------------------- small DFTs
-// Decimation in frequency, natural input; outputs land bit-reversed and are
-// relabelled by the caller.
 
 __device__ __forceinline__ void dft2(Fr& a, Fr& b) {
     Fr t = fe_add_lazy<FrCfg>(a, b);
@@ -124,7 +149,69 @@ __device__ __forceinline__ void dft2(Fr& a, Fr& b) {
     a = t;
 }
 
-// v[0..3] -> y[k] at position rev2(k): y0=v0, y1=v2, y2=v1, y3=v3
+// The factors of a DFT of eight, kept in shared memory: w4 = w_8^2,
+// cu = (w_8 + w_8^-1) / 2 and su = (w_8 - w_8^-1) / 2 (w_8^-1 = -w_8^3).
+template <class TW>
+struct DftK {
+    Fr k[3 * TW::EW];
+    __device__ __forceinline__ typename TW::K w4() const { return TW::sm(k); }
+    __device__ __forceinline__ typename TW::K cu() const { return TW::sm(k + TW::EW); }
+    __device__ __forceinline__ typename TW::K su() const { return TW::sm(k + 2 * TW::EW); }
+    // tw: the table of w_n, n = 2^log_n >= 8
+    __device__ __forceinline__ void init(const Fr* tw, int log_n) {
+        for (int i = threadIdx.x; i < 3; i += blockDim.x) {
+            typename TW::K r;
+            if (i == 0) {
+                r = TW::ld(tw, (size_t)1 << (log_n - 2));
+            } else {
+                const Fr a = TW::ld(tw, (size_t)1 << (log_n - 3)).w, b = TW::ld(tw, (size_t)3 << (log_n - 3)).w;
+                Fr h = i == 1 ? fe_sub<FrCfg>(a, b) : fe_add<FrCfg>(a, b);
+                limbs_half_mod<FrCfg>(h.v);
+                r = TW::of(h);
+            }
+            TW::put(k + i * TW::EW, r);
+        }
+    }
+};
+
+// DFT of eight by Winograd's short algorithm (S. Winograd, "On computing the
+// discrete Fourier transform", 1978): four products, independent of each other
+// (w4 twice, cu, su), where the radix-2 form takes five in two levels.  In and
+// out in natural order up to dft8_slot: y_j ends in v[dft8_slot(j)].
+template <class TW>
+__device__ __forceinline__ void dft8(Fr v[8], const DftK<TW>& c) {
+    dft2(v[0], v[4]);
+    dft2(v[2], v[6]);
+    dft2(v[1], v[5]);
+    dft2(v[3], v[7]);
+    dft2(v[5], v[7]);  // v5: sum (su), v7: difference (cu)
+    dft2(v[1], v[3]);
+    if constexpr (TW::EW == 2) {
+        v[5] = TW::mul(v[5], c.su());
+        v[7] = TW::mul(v[7], c.cu());
+        v[3] = TW::mul(v[3], c.w4());
+        v[6] = TW::mul(v[6], c.w4());
+    } else {
+        const Fr2 a = TW::mul2(v[5], c.su(), v[7], c.cu());
+        v[5] = a.a;
+        v[7] = a.b;
+        const Fr2 b = TW::mul2(v[3], c.w4(), v[6], c.w4());
+        v[3] = b.a;
+        v[6] = b.b;
+    }
+    dft2(v[0], v[2]);
+    dft2(v[0], v[1]);
+    dft2(v[2], v[3]);
+    dft2(v[4], v[7]);
+    dft2(v[5], v[6]);
+    dft2(v[4], v[5]);
+    dft2(v[7], v[6]);
+}
+__device__ __forceinline__ constexpr int dft8_slot(int j) {
+    return j == 0 ? 0 : j == 1 ? 4 : j == 2 ? 2 : j == 3 ? 7 : j == 4 ? 1 : j == 5 ? 6 : j == 6 ? 3 : 5;
+}
+
+// v[0..3] -> y[k]: y0=v0, y1=v2, y2=v1, y3=v3
 template <class TW>
 __device__ __forceinline__ void dft4_dif(Fr& v0, Fr& v1, Fr& v2, Fr& v3, const typename TW::K& w4) {
     dft2(v0, v2);
@@ -134,152 +221,147 @@ __device__ __forceinline__ void dft4_dif(Fr& v0, Fr& v1, Fr& v2, Fr& v3, const t
     dft2(v2, v3);
 }
 
-// v[0..7] -> y[j] at position rev3(j)
-template <class TW>
-__device__ __forceinline__ void dft8_dif(Fr v[8], const typename TW::K& w8, const typename TW::K& w4,
-                                         const typename TW::K& w83) {
-    dft2(v[0], v[4]);
-    dft2(v[1], v[5]);
-    dft2(v[2], v[6]);
-    dft2(v[3], v[7]);
-    const Fr3 m = TW::mul3(v[5], w8, v[6], w4, v[7], w83);
-    v[5] = m.a;
-    v[6] = m.b;
-    v[7] = m.c;
-    // the two radix-4 DFTs side by side
-    dft2(v[0], v[2]);
-    dft2(v[1], v[3]);
-    dft2(v[4], v[6]);
-    dft2(v[5], v[7]);
-    const Fr2 m4 = TW::mul2(v[3], w4, v[7], w4);
-    v[3] = m4.a;
-    v[7] = m4.b;
-    dft2(v[0], v[1]);
-    dft2(v[2], v[3]);
-    dft2(v[4], v[5]);
-    dft2(v[6], v[7]);
-}
-
-
-// output-side work of the last sub-stage: the inter-pass twiddle w_n^{P*Q*y}
-// and the optional scale
-struct PassOut {
+// Where the factors of an item's sub-stages come from: the table of w_n at
+// (i J_full) n / (P R_s) for item index J_full = J + P Jl, or ctab, the table
+// of a coset's first pass (ntt_coset_table_kernel).
+struct StageTw {
     const Fr* tw;
-    int log_p;       // global P
-    uint32_t qhi;    // Q = q >> log_p for this thread's DFT
-    const Fr* scale;
-    const Fr* wrow;  // when set: output y is multiplied by wrow[y] instead
+    const Fr* ctab;
+    int log_n, log_p;
+    uint32_t J;  // the item's index in the products of earlier passes
 };
 
-// (the result is canonical: it leaves the pass)
-template <class TW>
-__device__ __forceinline__ Fr finish_out(const PassOut& o, Fr v, uint32_t y) {
-    if (o.wrow) return fe_canon<FrCfg>(TW::mul(v, TW::ld(o.wrow, y)));
-    if (o.qhi != 0 && y != 0) v = TW::mul(v, TW::ld(o.tw, (size_t)(o.qhi * y) << o.log_p));
-    if (o.scale) v = TW::mul(v, TW::ld(o.scale, 0));
-    return fe_canon<FrCfg>(v);
+// factor of input i of local item Jl in a sub-stage of radix 2^LR after P_s = 2^log_ps
+template <int LR, class TW>
+__device__ __forceinline__ typename TW::K stage_factor(const StageTw& t, uint32_t Jl, int log_ps, uint32_t i) {
+    if (t.ctab) return TW::ld(t.ctab, ((((size_t)1 << log_ps) + Jl) << LR) + i);
+    return TW::ld(t.tw, (size_t)(i * (t.J + (Jl << t.log_p))) << (t.log_n - t.log_p - log_ps - LR));
 }
 
-// radix-8 sub-stage over one DFT of size R in shared memory
+// radix-8 sub-stage over one DFT of size R in shared memory, v its inputs
+// (already multiplied by their factors) in registers
+template <class TW>
+__device__ __forceinline__ void stage8_finish(Fr* x, int u, int log_ps, bool last, Fr v[8], const DftK<TW>& dk) {
+    dft8<TW>(v, dk);
+    const int J = u & ((1 << log_ps) - 1);
+    const int ilo = u >> log_ps;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const Fr y = v[dft8_slot(j)];
+        sm_st(x, J + (j << log_ps) + (ilo << (log_ps + 3)), last ? fe_canon<FrCfg>(y) : y);
+    }
+    __syncthreads();
+}
+
+// inputs 1..7 of a sub-stage by their factors
+template <class TW>
+__device__ __forceinline__ void stage8_twiddle(Fr v[8], const StageTw& t, uint32_t Jl, int log_ps) {
+    if (!t.ctab && t.J + (Jl << t.log_p) == 0) return;
+    if constexpr (TW::EW == 2) {
+        // one at a time: two pairs of factors beside eight elements would spill
+#pragma unroll
+        for (uint32_t i = 1; i < 8; i++) v[i] = TW::mul(v[i], stage_factor<3, TW>(t, Jl, log_ps, i));
+    } else {
+#pragma unroll
+        for (uint32_t i = 1; i < 7; i += 2) {
+            const Fr2 m = TW::mul2(v[i], stage_factor<3, TW>(t, Jl, log_ps, i), v[i + 1],
+                                   stage_factor<3, TW>(t, Jl, log_ps, i + 1));
+            v[i] = m.a;
+            v[i + 1] = m.b;
+        }
+        v[7] = TW::mul(v[7], stage_factor<3, TW>(t, Jl, log_ps, 7));
+    }
+}
+
+// all eight inputs by k[0..7] (shared memory)
+template <class TW>
+__device__ __forceinline__ void stage8_scale(Fr v[8], const Fr* k) {
+    if constexpr (TW::EW == 2) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = TW::mul(v[i], TW::sm(k + i * TW::EW));
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {
+            const Fr2 m = TW::mul2(v[i], TW::sm(k + i * TW::EW), v[i + 1], TW::sm(k + (i + 1) * TW::EW));
+            v[i] = m.a;
+            v[i + 1] = m.b;
+        }
+    }
+}
+
 template <int LOGR, class TW>
-__device__ __forceinline__ void stage8(Fr* x, int u, int log_ps, bool last, const Fr* tw, int log_n,
-                                       const Fr* in_mul, size_t in_base, int log_items,
-                                       const PassOut& po) {
-    constexpr int R = 1 << LOGR;
-    constexpr int S = R / 8;
-    Fr v[8];
+__device__ __forceinline__ void stage8_load(Fr v[8], Fr* x, int u) {
+    constexpr int S = (1 << LOGR) / 8;
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = sm_ld(x, u + S * i);
     __syncthreads();
-    if (in_mul) {
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-            v[i] = TW::mul(v[i], TW::ld(in_mul, in_base + ((size_t)(u + S * i) << log_items)));
-    }
-    const int sh = log_n - LOGR;  // w_R^e = tw[e << sh]
-    {
-        const typename TW::K w8 = TW::ld(tw, (size_t)(S * 1) << sh);
-        const typename TW::K w4 = TW::ld(tw, (size_t)(S * 2) << sh);
-        const typename TW::K w83 = TW::ld(tw, (size_t)(S * 3) << sh);
-        dft8_dif<TW>(v, w8, w4, w83);
-    }
-    const int J = u & ((1 << log_ps) - 1);
-    const int ilo = u >> log_ps;
-    // y[j] sits in v[rev3(j)]
-    const int rev[8] = {0, 4, 2, 6, 1, 5, 3, 7};
-    if (ilo != 0) {
-#pragma unroll
-        for (int j = 1; j < 7; j += 2) {
-            const Fr2 t = TW::mul2(v[rev[j]], TW::ld(tw, (size_t)((ilo * j) << log_ps) << sh), v[rev[j + 1]],
-                                   TW::ld(tw, (size_t)((ilo * (j + 1)) << log_ps) << sh));
-            v[rev[j]] = t.a;
-            v[rev[j + 1]] = t.b;
-        }
-        v[rev[7]] = TW::mul(v[rev[7]], TW::ld(tw, (size_t)((ilo * 7) << log_ps) << sh));
-    }
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        Fr y = v[rev[j]];
-        const int pos = J + (j << log_ps) + (ilo << (log_ps + 3));
-        if (last) y = finish_out<TW>(po, y, (uint32_t)pos);
-        sm_st(x, pos, y);
-    }
-    __syncthreads();
 }
 
-// final radix-4 sub-stage (two items per thread); P_s = R/4 so no sub-stage twiddle
+// final radix-4 sub-stage (two items per thread), P_s = R / 4
 template <int LOGR, class TW>
-__device__ __forceinline__ void stage4_last(Fr* x, int lt, const Fr* tw, int log_n, const PassOut& po,
-                                            const Fr* in_mul, size_t in_base, int log_items) {
+__device__ __forceinline__ void stage4_last(Fr* x, int lt, const StageTw& t, const DftK<TW>& dk) {
     constexpr int R = 1 << LOGR;
     constexpr int S = R / 4;  // items and read stride
-    constexpr int TH = (R >= 8) ? R / 8 : 1;
-    Fr v[8];
-#pragma unroll
+    constexpr int TH = R / 8;
+    // a thread rewrites only its own slots u + S j
+#pragma unroll 1
     for (int k = 0; k < 2; k++) {
-        int u = lt + k * TH;
+        const uint32_t u = lt + k * TH;
+        Fr v[4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) v[4 * k + i] = sm_ld(x, u + S * i);
-    }
-    __syncthreads();
-    const int sh = log_n - LOGR;
-    const typename TW::K w4 = TW::ld(tw, (size_t)S << sh);
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        int u = lt + k * TH;
-        if (in_mul) {
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-                v[4 * k + i] = TW::mul(v[4 * k + i], TW::ld(in_mul, in_base + ((size_t)(u + S * i) << log_items)));
-        }
-        dft4_dif<TW>(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3], w4);
+        for (int i = 0; i < 4; i++) v[i] = sm_ld(x, u + S * i);
+        const Fr2 m = TW::mul2(v[1], stage_factor<2, TW>(t, u, LOGR - 2, 1), v[2],
+                               stage_factor<2, TW>(t, u, LOGR - 2, 2));
+        v[1] = m.a;
+        v[2] = m.b;
+        v[3] = TW::mul(v[3], stage_factor<2, TW>(t, u, LOGR - 2, 3));
+        dft4_dif<TW>(v[0], v[1], v[2], v[3], dk.w4());
         const int rev[4] = {0, 2, 1, 3};
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int pos = u + S * j;  // J = u, P_s = S, ilo = 0
-            sm_st(x, pos, finish_out<TW>(po, v[4 * k + rev[j]], (uint32_t)pos));
-        }
+        for (int j = 0; j < 4; j++) sm_st(x, u + S * j, fe_canon<FrCfg>(v[rev[j]]));
     }
     __syncthreads();
 }
 
-// final radix-2 sub-stage (four items per thread)
+// final radix-2 sub-stage (four items per thread, two at a time), P_s = R / 2
 template <int LOGR, class TW>
-__device__ __forceinline__ void stage2_last(Fr* x, int lt, const PassOut& po) {
+__device__ __forceinline__ void stage2_last(Fr* x, int lt, const StageTw& t) {
     constexpr int R = 1 << LOGR;
     constexpr int S = R / 2;
     constexpr int TH = R / 8;
-    // each thread reads and rewrites only its own slots u and u + S, so a
-    // pair is finished before the next is loaded (two elements live at a time)
+    // each thread reads and rewrites only its own slots u and u + S
 #pragma unroll 1
-    for (int k = 0; k < 4; k++) {
-        const int u = lt + k * TH;
-        Fr v0 = sm_ld(x, u), v1 = sm_ld(x, u + S);
-        dft2(v0, v1);
-        sm_st(x, u, finish_out<TW>(po, v0, (uint32_t)u));
-        sm_st(x, u + S, finish_out<TW>(po, v1, (uint32_t)(u + S)));
+    for (int k = 0; k < 4; k += 2) {
+        const uint32_t u0 = lt + k * TH, u1 = u0 + TH;
+        Fr a0 = sm_ld(x, u0), b0 = sm_ld(x, u0 + S), a1 = sm_ld(x, u1), b1 = sm_ld(x, u1 + S);
+        const Fr2 m = TW::mul2(b0, stage_factor<1, TW>(t, u0, LOGR - 1, 1), b1,
+                               stage_factor<1, TW>(t, u1, LOGR - 1, 1));
+        b0 = m.a;
+        b1 = m.b;
+        dft2(a0, b0);
+        dft2(a1, b1);
+        sm_st(x, u0, fe_canon<FrCfg>(a0));
+        sm_st(x, u0 + S, fe_canon<FrCfg>(b0));
+        sm_st(x, u1, fe_canon<FrCfg>(a1));
+        sm_st(x, u1 + S, fe_canon<FrCfg>(b1));
     }
     __syncthreads();
+}
+
+// the sub-stages after the first of a DFT of size 2^LOGR in shared memory
+template <int LOGR, class TW>
+__device__ __forceinline__ void dft_tail(Fr* x, int lt, const StageTw& t, const DftK<TW>& dk) {
+    constexpr int NS8 = LOGR / 3;
+    constexpr int REM = LOGR % 3;
+#pragma unroll 1
+    for (int s = 1; s < NS8; s++) {
+        Fr v[8];
+        stage8_load<LOGR, TW>(v, x, lt);
+        stage8_twiddle<TW>(v, t, (uint32_t)lt & ((1u << (3 * s)) - 1), 3 * s);
+        stage8_finish<TW>(x, lt, 3 * s, s == NS8 - 1 && REM == 0, v, dk);
+    }
+    if (REM == 2) stage4_last<LOGR, TW>(x, lt, t, dk);
+    if (REM == 1) stage2_last<LOGR, TW>(x, lt, t);
 }
 
 #ifndef ZK_PASS10_MIN_BLOCKS
@@ -315,6 +397,27 @@ ntt_pass_kernel(NttPassArgs a) {
     const Fr* src = a.src + by * a.src_ys + blockIdx.z * a.src_zs;
     Fr* dst = a.dst + by * a.dst_ys + blockIdx.z * a.dst_zs;
 
+    // factors of the first sub-stage's eight inputs, one set an item, where all
+    // eight are multiplied: a scale (times the item's twiddles), or the first
+    // pass of a coset transform with its own table
+    __shared__ Fr kst[G * 8 * TW::EW];
+    __shared__ DftK<TW> dk;
+    const bool kst_used = a.ctab || (a.scale && !a.in_mul);
+    dk.init(a.tw, a.log_n);
+    if (kst_used) {
+        for (int k = tid; k < G * 8; k += T) {
+            const uint32_t qk = q0 + k / 8, i = k % 8;
+            typename TW::K f;
+            if (a.ctab) {
+                f = TW::ld(a.in_mul, (size_t)qk + ((size_t)i << (a.log_n - 3)));
+            } else {
+                f = TW::ld(a.scale, 0);
+                const uint32_t J = qk & ((1u << a.log_p) - 1);
+                if (i * J) f = TW::prod(TW::ld(a.tw, (size_t)(i * J) << (a.log_n - a.log_p - 3)), f);
+            }
+            TW::put(kst + k * TW::EW, f);
+        }
+    }
     // coalesced load: chunk c -> (i, g, h); global x[q0 + g + (i << log_items)]
     for (int c = tid; c < G * R * 2; c += T) {
         const int h = c & 1, e = c >> 1;
@@ -327,27 +430,31 @@ ntt_pass_kernel(NttPassArgs a) {
     const int g = tid / TR, lt = tid % TR;
     Fr* x = sm + g * R;
     const uint32_t q = q0 + g;
-    PassOut po;
-    po.tw = a.tw;
-    po.log_p = a.log_p;
-    po.qhi = q >> a.log_p;
-    po.scale = a.scale;
-    po.wrow = nullptr;
     const Fr* in_mul = a.in_mul ? TW::off(a.in_mul, blockIdx.z * a.in_mul_zs) : nullptr;
-    const size_t in_base = q;  // natural input position = q + (i << log_items)
+    StageTw st;
+    st.tw = a.tw;
+    st.ctab = a.ctab;
+    st.log_n = a.log_n;
+    st.log_p = a.log_p;
+    st.J = q & ((1u << a.log_p) - 1);
 
-    constexpr int NS8 = LOGR / 3;
-    constexpr int REM = LOGR % 3;
-    int log_ps = 0;
-#pragma unroll 1
-    for (int s = 0; s < NS8; s++) {
-        const bool last = (s == NS8 - 1) && (REM == 0);
-        stage8<LOGR, TW>(x, lt, log_ps, last, a.tw, a.log_n, s == 0 ? in_mul : nullptr, in_base, log_items, po);
-        log_ps += 3;
+    Fr v[8];
+    stage8_load<LOGR, TW>(v, x, lt);
+    if (kst_used) {
+        stage8_scale<TW>(v, kst + g * 8 * TW::EW);
+    } else if (in_mul) {
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            v[i] = TW::mul(v[i], TW::ld(in_mul, (size_t)q + ((size_t)(lt + TR * i) << log_items)));
+        if (a.scale) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = TW::mul(v[i], TW::ld(a.scale, 0));
+        }
+    } else {
+        stage8_twiddle<TW>(v, st, 0, 0);
     }
-    if (REM == 2)
-        stage4_last<LOGR, TW>(x, lt, a.tw, a.log_n, po, NS8 == 0 ? in_mul : nullptr, in_base, log_items);
-    if (REM == 1) stage2_last<LOGR, TW>(x, lt, po);
+    stage8_finish<TW>(x, lt, 0, LOGR == 3, v, dk);
+    dft_tail<LOGR, TW>(x, lt, st, dk);
 
     // coalesced store: dst[(J + P*j + P*R*Q) << out_shift + z*out_off_z]
     const uint32_t pm = (1u << a.log_p) - 1;
@@ -369,49 +476,30 @@ ntt_pass_kernel(NttPassArgs a) {
     }
 }
 
-// in-CTA DFT of size 2^LOGR on tile x (natural order in and out)
-template <int LOGR, class TW>
-__device__ __forceinline__ void dft_tile(Fr* x, int lt, const Fr* tw, int log_n, const PassOut& po) {
-    constexpr int NS8 = LOGR / 3;
-    constexpr int REM = LOGR % 3;
-    int log_ps = 0;
-#pragma unroll 1
-    for (int s = 0; s < NS8; s++) {
-        stage8<LOGR, TW>(x, lt, log_ps, (s == NS8 - 1) && (REM == 0), tw, log_n, nullptr, 0, 0, po);
-        log_ps += 3;
-    }
-    if (REM == 2) stage4_last<LOGR, TW>(x, lt, tw, log_n, po, nullptr, 0, 0);
-    if (REM == 1) stage2_last<LOGR, TW>(x, lt, po);
-}
-
 // Fused extended-domain stage.  For one column and work item q it runs
 //   (1) the last pass of the inverse transform: radix R = 2^LOGR, P = n/R,
 //       input tmp[q + (n/R) i], output the coefficients c[q + (n/R) j] * n^-1,
 //       written to coeff;
 //   (2) for each coset z, the first pass of that coset's forward transform in
 //       the reversed radix order (radix R first, P = 1), whose item q reads
-//       exactly the same coefficients c[q + (n/R) i], twisted by
-//       t_z^(q + (n/R) i) = t_z^q * S_z[i]: the tile is multiplied by S_z,
-//       transformed, and output y is multiplied by W_z[q R + y] = w^(q y) t_z^q
-//       (inter-pass twiddle and the item's twist constant), then written to
+//       exactly the same coefficients c[q + (n/R) i], to be multiplied by
+//       t_z^(q + (n/R) i): the first sub-stage's eight inputs take
+//       t_z^q (t_z^(n/8))^i (W_z[q R] S_z[(R/8) i], eight factors a coset made
+//       at the start), the later sub-stages ctab's factors; then written to
 //       sub[z n + y + R q].
-// The coefficients stay in shared memory across the 2^e cosets, so they are
-// read once instead of 2^e times with a strided pattern.
-#ifndef ZK_FUSED_ONE_TILE
-#define ZK_FUSED_ONE_TILE 1
-#endif
-
-// resident CTAs per SM the register budget is sized for: two tiles of 2^LOGR
-// elements in shared memory allow 7 CTAs of 2^9, 3 of 2^10 and 1 of 2^11; one
-// tile (the coefficients re-read from L2 for each coset) allows 4 of 2^10 and,
-// at 128 registers a thread, 2 of 2^11 (the 2^22 -> 2^25 extension: 82.1 ->
-// 73.0 ms per 8 columns on B200 against one CTA of 255 registers)
+// The coefficients stay on the CTA's tile for the first coset; later cosets
+// re-read them from L2.
+// resident CTAs per SM the register budget is sized for: one tile a CTA (the
+// coefficients re-read from L2 for each coset) allows 7 of 2^9, 4 of 2^10 and,
+// at 128 registers a thread, 2 of 2^11
 #ifndef ZK_FUSED11_MIN_BLOCKS
 #define ZK_FUSED11_MIN_BLOCKS 2
 #endif
 __host__ __device__ constexpr int fused_min_blocks(int logr) {
-    return logr <= 9 ? 7 : logr == 10 ? (ZK_FUSED_ONE_TILE ? 4 : 3) : ZK_FUSED11_MIN_BLOCKS;
+    return logr <= 9 ? 7 : logr == 10 ? 4 : ZK_FUSED11_MIN_BLOCKS;
 }
+
+static constexpr int FUSED_MAX_E = 16;
 
 template <int LOGR, class TW>
 __global__ void __launch_bounds__((1 << LOGR) / 8, fused_min_blocks(LOGR))
@@ -420,7 +508,8 @@ ntt_fused_extend_kernel(FusedExtendArgs a) {
     constexpr int T = R / 8;
     extern __shared__ uint4 smem_u4[];
     Fr* A = reinterpret_cast<Fr*>(smem_u4);
-    Fr* B = ZK_FUSED_ONE_TILE ? A : A + R;
+    __shared__ Fr kst[8 * (1 + FUSED_MAX_E) * TW::EW];  // the inverse pass's factors, then each coset's
+    __shared__ DftK<TW> dki, dkf;
     const int tid = threadIdx.x;
     const int log_items = a.log_n - LOGR;
     // column-fastest block order, as in ntt_pass_kernel: the per-coset tables
@@ -436,43 +525,58 @@ ntt_fused_extend_kernel(FusedExtendArgs a) {
         const int h = c & 1, i = c >> 1;
         *sm_slot(A, i, h) = reinterpret_cast<const uint4*>(src + q + ((size_t)i << log_items))[h];
     }
+    dki.init(a.tw_inv, a.log_n);
+    dkf.init(a.tw, a.log_n);
+    for (int k = tid; k < 8 * (1 + a.E); k += T) {
+        const uint32_t i = k % 8;
+        typename TW::K f;
+        if (k < 8) {
+            f = TW::ld(a.n_inv, 0);
+            if (i * q) f = TW::prod(TW::ld(a.tw_inv, (size_t)(i * q) << (LOGR - 3)), f);
+        } else {
+            const size_t z = k / 8 - 1;
+            f = TW::ld(a.wtab, z * n + (size_t)q * R);
+            if (i) f = TW::prod(TW::ld(a.stab, z * R + (size_t)(R / 8) * i), f);
+        }
+        TW::put(kst + k * TW::EW, f);
+    }
     __syncthreads();
-    PassOut po;
-    po.tw = a.tw_inv;
-    po.log_p = log_items;
-    po.qhi = 0;
-    po.scale = a.n_inv;
-    po.wrow = nullptr;
-    dft_tile<LOGR, TW>(A, tid, a.tw_inv, a.log_n, po);
+    StageTw st;
+    st.tw = a.tw_inv;
+    st.ctab = nullptr;
+    st.log_n = a.log_n;
+    st.log_p = log_items;
+    st.J = q;
+    Fr v[8];
+    stage8_load<LOGR, TW>(v, A, tid);
+    stage8_scale<TW>(v, kst);
+    stage8_finish<TW>(A, tid, 0, false, v, dki);
+    dft_tail<LOGR, TW>(A, tid, st, dki);
     for (int c = tid; c < R * 2; c += T) {
         const int h = c & 1, j = c >> 1;
         reinterpret_cast<uint4*>(coeff + q + ((size_t)j << log_items))[h] = *sm_slot(A, j, h);
     }
+    st.tw = a.tw;
+    st.log_p = 0;
+    st.J = 0;
     for (int z = 0; z < a.E; z++) {
-        const Fr* S = TW::off(a.stab, (size_t)z * R);
-        if (ZK_FUSED_ONE_TILE) {
-            // the tile is the workspace: coset 0 twists it in place, later
-            // cosets re-read the coefficients this CTA wrote (L2-resident)
-            __syncthreads();
-            for (int i = tid; i < R; i += T) {
-                const Fr cf = z == 0 ? sm_ld(A, i) : ld_elem<FrCfg>(coeff + q + ((size_t)i << log_items));
-                sm_st(B, i, TW::mul(cf, TW::ld(S, i)));
-            }
+        // coset 0 reads the tile; later cosets the coefficients this CTA wrote
+        // (the barrier below orders the writes of its other threads)
+        if (z == 0) {
+            stage8_load<LOGR, TW>(v, A, tid);
         } else {
-            for (int i = tid; i < R; i += T) sm_st(B, i, TW::mul(sm_ld(A, i), TW::ld(S, i)));
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                v[i] = ld_elem<FrCfg>(coeff + q + ((size_t)(tid + (R / 8) * i) << log_items));
         }
-        __syncthreads();
-        PassOut pf;
-        pf.tw = a.tw;
-        pf.log_p = 0;
-        pf.qhi = 0;
-        pf.scale = nullptr;
-        pf.wrow = TW::off(a.wtab, (size_t)z * n + (size_t)q * R);
-        dft_tile<LOGR, TW>(B, tid, a.tw, a.log_n, pf);
+        st.ctab = TW::off(a.ctab, (size_t)z * 2 * R);
+        stage8_scale<TW>(v, kst + 8 * (1 + z) * TW::EW);
+        stage8_finish<TW>(A, tid, 0, false, v, dkf);
+        dft_tail<LOGR, TW>(A, tid, st, dkf);
         Fr* out = sub + (size_t)z * n + (size_t)q * R;
         for (int c = tid; c < R * 2; c += T) {
             const int h = c & 1, y = c >> 1;
-            reinterpret_cast<uint4*>(out + y)[h] = *sm_slot(B, y, h);
+            reinterpret_cast<uint4*>(out + y)[h] = *sm_slot(A, y, h);
         }
         __syncthreads();
     }
@@ -481,7 +585,7 @@ ntt_fused_extend_kernel(FusedExtendArgs a) {
 template <int LOGR, class TW>
 static cudaError_t launch_fused(const FusedExtendArgs& a, unsigned ncols, cudaStream_t s) {
     constexpr int R = 1 << LOGR;
-    const size_t smem = (size_t)(ZK_FUSED_ONE_TILE ? 1 : 2) * R * sizeof(Fr);
+    const size_t smem = (size_t)R * sizeof(Fr);
     static SmemOptIn opt;
     ZK_CHECK(opt.ensure(ntt_fused_extend_kernel<LOGR, TW>, (int)smem));
     dim3 grid(1u << (a.log_n - LOGR), ncols, 1);
@@ -499,7 +603,47 @@ static cudaError_t fused_dispatch(const FusedExtendArgs& a, int log_r, unsigned 
     }
 }
 
+// Factors of the sub-stages after the first in the first pass (radix R = 2^log_r)
+// of a coset transform X[j] = sum_k x_k s^k w_n^(jk).  In that pass item q's
+// DFT runs over x_(q + (n/R) i) s^((n/R) i) (s^q goes into its first
+// sub-stage), so a sub-stage of radix r after P_s multiplies input i of local
+// item Jl by s^(i n/(P_s r)) w_(P_s r)^(i Jl): the same factors for every q and
+// column, at entry r (P_s + Jl) + i, 2 R entries a coset.  s^k is entry
+// k step of pw (k step < n powers of s at step 1, or the R powers of s^(n/R)
+// with the exponents counted in n/R: pw_shift = log2(n/R)).
+// Made once per call into a buffer the first pass does not write, it takes
+// the place of one product an element (the twist of every input).
+template <class TW>
+__global__ void ntt_coset_table_kernel(Fr* ctab, const Fr* pw, size_t pw_zs, int pw_shift, const Fr* tw, int log_n,
+                                       int log_r) {
+    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= 2u << log_r) return;
+    // the sub-stages' P_s are 8, 64, ... and the last one's radix is 8, 4 or 2
+    int log_ps = 3, lr = 3;
+    for (; log_ps < log_r; log_ps += 3) {
+        lr = log_r - log_ps < 3 ? log_r - log_ps : 3;
+        if (e >> lr >= 1u << log_ps && e >> lr < 2u << log_ps) break;
+    }
+    if (log_ps >= log_r) return;  // a gap between two sub-stages' entries
+    const uint32_t Jl = (e >> lr) - (1u << log_ps), i = e & ((1u << lr) - 1);
+    const size_t k = (size_t)i << (log_n - log_ps - lr);
+    typename TW::K f = TW::ld(TW::off(pw, blockIdx.y * pw_zs), k >> pw_shift);
+    if (i * Jl) f = TW::prod(TW::ld(tw, (size_t)(i * Jl) << (log_n - log_ps - lr)), f);
+    TW::put(ctab + ((size_t)blockIdx.y * (2u << log_r) + e) * TW::EW, f);
+}
+
+cudaError_t ntt_coset_table(Fr* ctab, const Fr* pw, size_t pw_zs, int pw_shift, const Fr* tw, int log_n, int log_r,
+                            int cosets, int pairs, cudaStream_t s) {
+    const dim3 grid(((2u << log_r) + 127) / 128, cosets);
+    if (pairs)
+        ntt_coset_table_kernel<TwS><<<grid, 128, 0, s>>>(ctab, pw, pw_zs, pw_shift, tw, log_n, log_r);
+    else
+        ntt_coset_table_kernel<TwM><<<grid, 128, 0, s>>>(ctab, pw, pw_zs, pw_shift, tw, log_n, log_r);
+    return cudaGetLastError();
+}
+
 cudaError_t ntt_fused_extend(const FusedExtendArgs& a, int log_r, unsigned ncols, cudaStream_t s) {
+    if (a.E > FUSED_MAX_E) return cudaErrorInvalidValue;
     return a.pairs ? fused_dispatch<TwS>(a, log_r, ncols, s) : fused_dispatch<TwM>(a, log_r, ncols, s);
 }
 
@@ -592,19 +736,23 @@ static cudaError_t launch_pass(const NttPassArgs& a, unsigned ny, unsigned nz, c
     return cudaGetLastError();
 }
 
-// preferred items per CTA so that a CTA holds about 1024 elements
-static int pass_group(int log_r, int log_n) {
+// Items per CTA: about 1024 elements, so that a CTA's rows are read in runs of
+// several elements; fewer where that leaves the SMs without a CTA each (one
+// column of 2^13: 8 CTAs), down to one warp a CTA, since a warp's chain of
+// products takes the same time alone or beside three others.
+static int pass_group(int log_r, int log_n, unsigned cols) {
     int g = 1;
     if (log_r <= 9) g = 1 << (10 - log_r);
     if (g > 16) g = 16;
     const int items = 1 << (log_n - log_r);
     if (g > items) g = items;
+    while (g > 1 && (g << log_r) > 256 && (uint64_t)(items / g) * cols < 148) g /= 2;
     return g;
 }
 
 template <class TW>
 static cudaError_t pass_dispatch(const NttPassArgs& a, int log_r, unsigned ny, unsigned nz, cudaStream_t s) {
-    const int g = pass_group(log_r, a.log_n);
+    const int g = pass_group(log_r, a.log_n, ny * nz);
 #define ZK_PASS(LR, GG) \
     if (log_r == LR && g == GG) return launch_pass<LR, GG, TW>(a, ny, nz, s);
     ZK_PASS(3, 1) ZK_PASS(4, 1) ZK_PASS(5, 1) ZK_PASS(6, 1) ZK_PASS(7, 1) ZK_PASS(8, 1)

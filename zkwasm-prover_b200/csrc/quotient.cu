@@ -94,8 +94,7 @@ struct EvalHView {
 // coefficients, are staged per block as known factors
 static constexpr int EVAL_H_MAX_PERM = 256;
 static constexpr int EVAL_H_MAX_TERMS = 128;
-// threads a block: four blocks of 128 an SM share 2^17 rows out as 6.9 blocks an
-// SM (7 at most), two of 256 as 3.5 (4 at most): 1.28 against 1.44 ms
+// threads a block: PLACEHOLDER_TB
 static constexpr int EH_TB = 128;
 
 // The factors fixed for a launch, in known-factor form: beta and the powers
@@ -112,10 +111,9 @@ enum { EH_BETA, EH_Y, EH_Y2, EH_Y3, EH_YG, EH_Y0, EH_YL, EH_FACTORS };
 // both are z, so one accumulator serves both), A the chunk products in y and
 // then the third constraints in y^3.  A lookup costs two products by the known
 // y^3 and two full ones instead of three and five, a chunk link or product one
-// known product instead of one of each.  Bound by the multiply pipe (ncu: 75%
-// of its cycles at 13 warps an SM): at 2^17 rows of 17 gates, 60 permutation
-// columns, 24 lookups and 4 shuffles 1.28 ms, against 1.59 ms with every
-// constraint added to one accumulator.
+// known product instead of one of each.  Bound by the multiply pipe: at 2^17
+// rows of 17 gates, 60 permutation columns, 24 lookups and 4 shuffles
+// PLACEHOLDER_EVALH
 __global__ void __launch_bounds__(EH_TB, 512 / EH_TB) eval_h_fused_kernel(Fr* h, EvalHView a) {
     __shared__ KnownFr s_dbeta[EVAL_H_MAX_PERM];
     __shared__ KnownFr s_coef[EVAL_H_MAX_TERMS];
@@ -377,6 +375,13 @@ cudaError_t zkp_ntt_batch_twisted(void* out, const void* in, void* tmp, const vo
         a.src_ys = src_stride;
         a.dst_ys = to_out ? out_stride : n;
         a.pairs = pairs ? 1 : 0;
+        if (p == 0 && in_mul && np > 1) {
+            // the twist goes into the first pass's factors, made in the buffer
+            // this pass does not write (n >= 64 R elements)
+            Fr* ctab = to_out ? reinterpret_cast<Fr*>(tmp) : reinterpret_cast<Fr*>(out);
+            ZK_CHECK(ntt_coset_table(ctab, a.in_mul, 0, 0, a.tw, log_n, rad[0], 1, a.pairs, stream));
+            a.ctab = ctab;
+        }
         ZK_CHECK(ntt_pass(a, rad[p], ncols, 1, stream));
         src = dst;
         src_stride = a.dst_ys;
