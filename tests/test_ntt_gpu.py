@@ -96,6 +96,28 @@ def test_ntt_batch_columns(O, gpu, log_n, ncols):
         assert (got[c * n:(c + 1) * n] == O.ntt(a[c * n:(c + 1) * n], log_n)).all()
 
 
+# on both sides of the size up to which passes take two elements a thread, and
+# the smallest sizes of each radix there
+@pytest.mark.parametrize("log_n,ncols", [(7, 1), (8, 3), (9, 5), (10, 64), (10, 65), (11, 1), (12, 16), (12, 17),
+                                         (15, 2), (15, 3), (16, 1)])
+def test_ntt_short_passes(O, gpu, log_n, ncols):
+    H = gpu.host
+    n = 1 << log_n
+    a = O.rand_fr(n * ncols, 700 + log_n + ncols)
+    tw = H.generate_omega_buffers(_omega_mont(O, log_n), log_n)
+    tw_inv = H.generate_omega_buffers(_omega_mont(O, log_n, True), log_n)
+    div = H.to_device(O.fr(pow(n, -1, O.R_MOD)))
+    buf, tmp = H.to_device(a), H.empty_fr(n * ncols)
+    out = H.ntt_batch(buf, tmp, tw, log_n, ncols)
+    torch.cuda.synchronize()
+    got = H.to_host(out)
+    for c in (0, ncols - 1):
+        assert (got[c * n:(c + 1) * n] == O.ntt(a[c * n:(c + 1) * n], log_n)).all()
+    out = H.ntt_batch(out, tmp if out is buf else buf, tw_inv, log_n, ncols, div)
+    torch.cuda.synchronize()
+    assert (H.to_host(out) == a).all()
+
+
 # fused stage radices: 2^18 -> 2^9, 2^19 -> 2^9, 2^20 and 2^21 -> 2^10, 2^22 -> 2^11
 @pytest.mark.parametrize("pairs", [False, True])
 @pytest.mark.parametrize("log_n,ext_bits,ncols", [(4, 3, 2), (10, 3, 3), (13, 3, 2), (16, 2, 2),

@@ -53,6 +53,8 @@ cudaError_t ntt_fused_tables(Fr* wtab, Fr* stab, const Fr* tw, const Fr* shift, 
 // out[2i], out[2i+1] = (w, w') of the Montgomery-form factors in[i], i < n
 cudaError_t shoup_pairs(Fr* out, const Fr* in, size_t n, cudaStream_t s);
 int ntt_plan(int log_n, int radices[4]);
+// whether `transforms` transforms of 2^log_n take the passes for short work
+bool ntt_is_short(int log_n, uint64_t transforms);
 // Full transform of ncols columns (stride col_stride elements) by the twiddle
 // table tw; result in buf or tmp (*result_in_tmp), multiplied by *scale if given.
 cudaError_t ntt_run(Fr* buf, Fr* tmp, const Fr* tw, const Fr* scale, int log_n, unsigned ncols,
