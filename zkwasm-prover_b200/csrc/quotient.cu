@@ -44,6 +44,8 @@ static inline const zk::Fr* CFr(const void* p) { return reinterpret_cast<const z
 
 namespace zk {
 
+static __device__ __forceinline__ void prefetch_row(const Fr* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
 static __device__ __forceinline__ uint32_t rot_row(uint32_t i, int rot, uint32_t n) {
     return (uint32_t)((int64_t)i + rot) & (n - 1);
 }
@@ -194,6 +196,11 @@ __global__ void __launch_bounds__(EH_TB, 512 / EH_TB) eval_h_fused_kernel(Fr* h,
                 Fr R = ld_elem<FrCfg>(a.perm_z[j] + i);
                 const int end = c + a.perm_chunk_len < a.perm_cols_n ? c + a.perm_chunk_len : a.perm_cols_n;
                 for (; c < end; c++) {
+                    // the next column's values into L1 while this one's products run
+                    if (c + 1 < a.perm_cols_n) {
+                        prefetch_row(a.perm_cols[c + 1] + i);
+                        prefetch_row(a.perm_sigmas[c + 1] + i);
+                    }
                     const Fr v = fe_add_lazy<FrCfg>(ld_elem<FrCfg>(a.perm_cols[c] + i), gamma);
                     const Fr bs = mul_known(ld_elem<FrCfg>(a.perm_sigmas[c] + i), s_k[EH_BETA]);
                     L = fe_mul_lazy<FrCfg>(L, fe_add_lazy<FrCfg>(v, bs));
@@ -209,6 +216,12 @@ __global__ void __launch_bounds__(EH_TB, 512 / EH_TB) eval_h_fused_kernel(Fr* h,
         Fr a0 = fe_zero<FrCfg>();  // A_0 (and A_last while only lookups have been added)
         for (int k = 0; k < a.lookups; k++) {
             const Fr* const* q = a.lookup_cols + 4 * k;
+            if (k + 1 < a.lookups) {
+                prefetch_row(q[4] + i);
+                prefetch_row(q[5] + i);
+                prefetch_row(q[6] + i);
+                prefetch_row(q[7] + i);
+            }
             const Fr tb = fe_add_lazy<FrCfg>(ld_elem<FrCfg>(q[1] + i), beta);
             const Fr z = ld_elem<FrCfg>(q[3] + i);
             Fr u = fe_mul_lazy<FrCfg>(fe_sub_lazy<FrCfg>(ld_elem<FrCfg>(q[3] + rn), z), tb);
