@@ -29,6 +29,19 @@ void hc_mul(int which, uint64_t* out, const uint64_t* a, const uint64_t* b, long
     }
 }
 
+// op 0: a^2 without the final subtraction; 1: a b + c d likewise (operands up to 2m)
+void hc_sqr_mul2(int which, int op, uint64_t* out, const uint64_t* a, const uint64_t* b, const uint64_t* c,
+                 const uint64_t* d, long n) {
+    for (long i = 0; i < 4 * n; i += 4) {
+        if (which == 0)
+            st(out + i, op == 0 ? fe_sqr_lazy<FrCfg>(ld<FrCfg>(a + i))
+                                : fe_mul2_lazy<FrCfg>(ld<FrCfg>(a + i), ld<FrCfg>(b + i), ld<FrCfg>(c + i), ld<FrCfg>(d + i)));
+        else
+            st(out + i, op == 0 ? fe_sqr_lazy<FqCfg>(ld<FqCfg>(a + i))
+                                : fe_mul2_lazy<FqCfg>(ld<FqCfg>(a + i), ld<FqCfg>(b + i), ld<FqCfg>(c + i), ld<FqCfg>(d + i)));
+    }
+}
+
 void hc_add(int which, uint64_t* out, const uint64_t* a, const uint64_t* b, long n) {
     for (long i = 0; i < n; i++) {
         if (which == 0)

@@ -35,6 +35,7 @@ def hc():
         "hc_xyzz_to_jac": [P, P],
         "hc_glv_split": [P, P, P, P, ctypes.c_long],
         "hc_lazy": [ctypes.c_int, P, P, P, ctypes.c_long],
+        "hc_sqr_mul2": [ctypes.c_int, ctypes.c_int, P, P, P, P, P, ctypes.c_long],
         "hc_madd_lazy_chain": [P, P, P, ctypes.c_long],
         "hc_mul_shoup": [P, P, P, P, ctypes.c_long],
         "hc_glv_phi": [P, P, ctypes.c_long],
@@ -84,6 +85,25 @@ def test_lazy_inputs_below_2m(O, hc):
         ints = O.fr_ints if which == 0 else O.fq_ints
         assert ints(out) == [x * y % mod for x, y in zip(xs, ys)]
         assert all(O.limbs_to_int(out[i]) < mod for i in range(out.shape[0]))
+
+
+@pytest.mark.parametrize("which", [0, 1])
+def test_square_and_sum_of_products(O, hc, which):
+    """a^2 and a b + c d with one reduction, for operands up to 2m: congruent
+    to the exact values and below 2m."""
+    mod = O.R_MOD if which == 0 else O.Q_MOD
+    rng = random.Random(19)
+    edge = [0, 1, mod - 1, mod, mod + 1, 2 * mod - 1, (1 << 254) - 1, 0xffffffff, (1 << 224) - 1]
+    xs = [(a, b, c, d) for a in edge for b in edge for c in (0, mod, 2 * mod) for d in (1, 2 * mod)]
+    xs += [tuple(rng.randrange(2 * mod) for _ in range(4)) for _ in range(2000)]
+    cols = [np.stack([O.int_to_limbs(x[j]) for x in xs]) for j in range(4)]
+    rinv = pow(1 << 256, -1, mod)
+    out = np.empty_like(cols[0])
+    for op, exact in ((0, lambda a, b, c, d: a * a), (1, lambda a, b, c, d: a * b + c * d)):
+        hc.hc_sqr_mul2(which, op, _p(out), *[_p(c) for c in cols], len(xs))
+        for i, x in enumerate(xs):
+            got = O.limbs_to_int(out[i])
+            assert got < 2 * mod and (got - exact(*x) * rinv) % mod == 0, (op, x)
 
 
 def test_inverse_pow_from_mont(O, hc):

@@ -329,6 +329,217 @@ ZK_HD Fe<C> fe_mul_lazy(const Fe<C>& a, const Fe<C>& b) {
     return r;
 }
 
+// a b + c d, reduced as above: one reduction for two products.  For a, b, c, d
+// <= 2m the sum reduces to below (8 m^2 + m 2^256) / 2^256 < 2.52 m, so one
+// conditional subtraction of 2m returns it to [0, 2m).  The accumulators stay
+// below (4 m + m) 2^32 + 5 m < 2^288.
+template <class C>
+ZK_HD Fe<C> fe_mul2_lazy(const Fe<C>& a, const Fe<C>& b, const Fe<C>& c, const Fe<C>& d) {
+    uint32_t m[8], m2[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        m[j] = C::M(j);
+        m2[j] = (C::M(j) << 1) | (j ? C::M(j - 1) >> 31 : 0u);
+    }
+    uint32_t e[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    uint32_t o[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        chain4<0>(e, a.v, b.v[i]);
+        chain4<1>(o, a.v, b.v[i]);
+        chain4<0>(e, c.v, d.v[i]);
+        chain4<1>(o, c.v, d.v[i]);
+        const uint32_t q = e[0] * C::INV;
+        chain4<0>(e, m, q);
+        chain4<1>(o, m, q);
+        merge_shift(o, e);
+#pragma unroll
+        for (int j = 0; j < 9; j++) {
+            e[j] = o[j];
+            o[j] = 0;
+        }
+    }
+    uint32_t u[8];
+    const uint32_t br = sub8_borrow(u, e, m2);
+    Fe<C> r;
+    select8(r.v, br, e, u);
+    return r;
+}
+
+// acc[0 .. 2N) += x[0] b, x[2] b, ... (N products side by side), carry into
+// acc[2N]
+template <int N>
+ZK_HD void chain_n(uint32_t* acc, const uint32_t* x, uint32_t b) {
+#if defined(__CUDA_ARCH__)
+    if (N == 1)
+        asm("mad.lo.cc.u32  %0, %3, %4, %0;\n\t"
+            "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+            "addc.u32       %2, %2, 0;"
+            : "+r"(acc[0]), "+r"(acc[1]), "+r"(acc[2])
+            : "r"(x[0]), "r"(b));
+    if (N == 2)
+        asm("mad.lo.cc.u32  %0, %5, %7, %0;\n\t"
+            "madc.hi.cc.u32 %1, %5, %7, %1;\n\t"
+            "madc.lo.cc.u32 %2, %6, %7, %2;\n\t"
+            "madc.hi.cc.u32 %3, %6, %7, %3;\n\t"
+            "addc.u32       %4, %4, 0;"
+            : "+r"(acc[0]), "+r"(acc[1]), "+r"(acc[2]), "+r"(acc[3]), "+r"(acc[4])
+            : "r"(x[0]), "r"(x[2]), "r"(b));
+    if (N == 3)
+        asm("mad.lo.cc.u32  %0, %7, %10, %0;\n\t"
+            "madc.hi.cc.u32 %1, %7, %10, %1;\n\t"
+            "madc.lo.cc.u32 %2, %8, %10, %2;\n\t"
+            "madc.hi.cc.u32 %3, %8, %10, %3;\n\t"
+            "madc.lo.cc.u32 %4, %9, %10, %4;\n\t"
+            "madc.hi.cc.u32 %5, %9, %10, %5;\n\t"
+            "addc.u32       %6, %6, 0;"
+            : "+r"(acc[0]), "+r"(acc[1]), "+r"(acc[2]), "+r"(acc[3]), "+r"(acc[4]), "+r"(acc[5]), "+r"(acc[6])
+            : "r"(x[0]), "r"(x[2]), "r"(x[4]), "r"(b));
+    if (N == 4)
+        asm("mad.lo.cc.u32  %0, %9,  %13, %0;\n\t"
+            "madc.hi.cc.u32 %1, %9,  %13, %1;\n\t"
+            "madc.lo.cc.u32 %2, %10, %13, %2;\n\t"
+            "madc.hi.cc.u32 %3, %10, %13, %3;\n\t"
+            "madc.lo.cc.u32 %4, %11, %13, %4;\n\t"
+            "madc.hi.cc.u32 %5, %11, %13, %5;\n\t"
+            "madc.lo.cc.u32 %6, %12, %13, %6;\n\t"
+            "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"
+            "addc.u32       %8, %8, 0;"
+            : "+r"(acc[0]), "+r"(acc[1]), "+r"(acc[2]), "+r"(acc[3]), "+r"(acc[4]), "+r"(acc[5]), "+r"(acc[6]),
+              "+r"(acc[7]), "+r"(acc[8])
+            : "r"(x[0]), "r"(x[2]), "r"(x[4]), "r"(x[6]), "r"(b));
+#else
+    uint64_t c = 0;
+    for (int k = 0; k < N; k++) {
+        const uint64_t p = (uint64_t)x[2 * k] * b;
+        uint64_t s = (uint64_t)acc[2 * k] + (uint32_t)p + c;
+        acc[2 * k] = (uint32_t)s;
+        c = s >> 32;
+        s = (uint64_t)acc[2 * k + 1] + (uint32_t)(p >> 32) + c;
+        acc[2 * k + 1] = (uint32_t)s;
+        c = s >> 32;
+    }
+    acc[2 * N] = (uint32_t)(acc[2 * N] + c);
+#endif
+}
+
+// r[0..8) += x[0..8) with carry in c, returns the carry
+ZK_HD uint32_t add8_in(uint32_t* r, const uint32_t* x, uint32_t c) {
+#if defined(__CUDA_ARCH__)
+    uint32_t co;
+    asm("add.cc.u32  %8, %17, 0xffffffff;\n\t"
+        "addc.cc.u32 %0, %0, %9;\n\t"
+        "addc.cc.u32 %1, %1, %10;\n\t"
+        "addc.cc.u32 %2, %2, %11;\n\t"
+        "addc.cc.u32 %3, %3, %12;\n\t"
+        "addc.cc.u32 %4, %4, %13;\n\t"
+        "addc.cc.u32 %5, %5, %14;\n\t"
+        "addc.cc.u32 %6, %6, %15;\n\t"
+        "addc.cc.u32 %7, %7, %16;\n\t"
+        "addc.u32    %8, 0, 0;"
+        : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "=&r"(co)
+        : "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(x[3]), "r"(x[4]), "r"(x[5]), "r"(x[6]), "r"(x[7]), "r"(c));
+    return co;
+#else
+    uint64_t s = c;
+    for (int j = 0; j < 8; j++) {
+        s += (uint64_t)r[j] + x[j];
+        r[j] = (uint32_t)s;
+        s >>= 32;
+    }
+    return (uint32_t)s;
+#endif
+}
+
+// t[0..16) += the squares a_i^2 side by side (no carry out)
+ZK_HD void add_squares(uint32_t t[16], const uint32_t a[8]) {
+#if defined(__CUDA_ARCH__)
+    asm("mad.lo.cc.u32  %0, %16, %16, %0;\n\t"
+        "madc.hi.cc.u32 %1, %16, %16, %1;\n\t"
+        "madc.lo.cc.u32 %2, %17, %17, %2;\n\t"
+        "madc.hi.cc.u32 %3, %17, %17, %3;\n\t"
+        "madc.lo.cc.u32 %4, %18, %18, %4;\n\t"
+        "madc.hi.cc.u32 %5, %18, %18, %5;\n\t"
+        "madc.lo.cc.u32 %6, %19, %19, %6;\n\t"
+        "madc.hi.cc.u32 %7, %19, %19, %7;\n\t"
+        "madc.lo.cc.u32 %8, %20, %20, %8;\n\t"
+        "madc.hi.cc.u32 %9, %20, %20, %9;\n\t"
+        "madc.lo.cc.u32 %10, %21, %21, %10;\n\t"
+        "madc.hi.cc.u32 %11, %21, %21, %11;\n\t"
+        "madc.lo.cc.u32 %12, %22, %22, %12;\n\t"
+        "madc.hi.cc.u32 %13, %22, %22, %13;\n\t"
+        "madc.lo.cc.u32 %14, %23, %23, %14;\n\t"
+        "madc.hi.u32    %15, %23, %23, %15;"
+        : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]), "+r"(t[8]),
+          "+r"(t[9]), "+r"(t[10]), "+r"(t[11]), "+r"(t[12]), "+r"(t[13]), "+r"(t[14]), "+r"(t[15])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]));
+#else
+    uint64_t c = 0;
+    for (int i = 0; i < 8; i++) {
+        const uint64_t p = (uint64_t)a[i] * a[i];
+        c += (uint64_t)t[2 * i] + (uint32_t)p;
+        t[2 * i] = (uint32_t)c;
+        c >>= 32;
+        c += (uint64_t)t[2 * i + 1] + (uint32_t)(p >> 32);
+        t[2 * i + 1] = (uint32_t)c;
+        c >>= 32;
+    }
+#endif
+}
+
+// a^2 2^-256 mod m for a < 2m, below 2m: the 28 products of different limbs
+// once, in even and odd chains like the product's, doubled, the eight squares
+// added, then the low half reduced by rows and the high half added: 100 wide
+// multiply-adds where the product takes 128, for about 45 more additions.
+template <class C>
+ZK_HD Fe<C> fe_sqr_lazy(const Fe<C>& a) {
+    const uint32_t* x = a.v;
+    uint32_t O[17], E[17], t[16];
+#pragma unroll
+    for (int k = 0; k < 17; k++) O[k] = E[k] = 0;
+    chain_n<4>(O + 1, x + 1, x[0]);
+    chain_n<3>(E + 2, x + 2, x[0]);
+    chain_n<3>(O + 3, x + 2, x[1]);
+    chain_n<3>(E + 4, x + 3, x[1]);
+    chain_n<3>(O + 5, x + 3, x[2]);
+    chain_n<2>(E + 6, x + 4, x[2]);
+    chain_n<2>(O + 7, x + 4, x[3]);
+    chain_n<2>(E + 8, x + 5, x[3]);
+    chain_n<2>(O + 9, x + 5, x[4]);
+    chain_n<1>(E + 10, x + 6, x[4]);
+    chain_n<1>(O + 11, x + 6, x[5]);
+    chain_n<1>(E + 12, x + 7, x[5]);
+    chain_n<1>(O + 13, x + 7, x[6]);
+    const uint32_t c = add8_in(O, E, 0);
+    add8_in(O + 8, E + 8, c);
+#pragma unroll
+    for (int k = 0; k < 16; k++) t[k] = k ? (O[k] << 1) | (O[k - 1] >> 31) : O[0] << 1;
+    add_squares(t, x);
+    uint32_t m[8];
+    uint32_t e[9], o[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        m[j] = C::M(j);
+        e[j] = t[j];
+    }
+    e[8] = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const uint32_t q = e[0] * C::INV;
+        chain4<0>(e, m, q);
+        chain4<1>(o, m, q);
+        merge_shift(o, e);
+#pragma unroll
+        for (int j = 0; j < 9; j++) {
+            e[j] = o[j];
+            o[j] = 0;
+        }
+    }
+    Fe<C> r;
+    add8_carry(r.v, e, t + 8);
+    return r;
+}
+
 // ---------------------------------------------------------------------------
 // Products by a known factor (Shoup): for a canonical w and its companion
 // w' = floor(w 2^256 / m), a * w mod m for any a < 2^256 from q = the high
