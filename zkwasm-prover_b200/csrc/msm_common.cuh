@@ -40,7 +40,7 @@ __device__ __forceinline__ void st_xyzz(Xyzz* p, const Xyzz& v) {
 // its own takes fourteen and nine, and a warp runs eight of them side by side.
 // All 32 lanes call these functions.  Coordinates lie in [0, 2p); ZZ of the
 // identity is zero itself, as are its other components.  Alone on a
-// sub-partition a quad addition takes 4400 clocks and a doubling 3250, a lane's
+// sub-partition a quad addition takes 4400 clocks and a doubling 2800, a lane's
 // own addition 13100 and doubling 8700 (a product is 850-900 clocks of latency).
 
 static constexpr int COOP_THREADS = 32;
@@ -78,19 +78,19 @@ __device__ __forceinline__ void qd_store(Xyzz* p, const Fq& v) {
 __device__ __forceinline__ Fq qd_dbl(const Fq& p) {
     const int k = qd_lane();
     // X^2, V = Y^2; M = 3/2 X^2
-    const Fq r = cmul_lazy(p, p);
+    const Fq r = fe_mul_lazy<FqCfg>(p, p);
     Fq h = r;
     limbs_half_mod<FqCfg>(h.v);
     h = fe_add_lazy<FqCfg>(r, h);
     const Fq V = qd_shfl(r, 1), M = qd_shfl(h, 0);
     // S = X V, W = Y V, ZZ3 = ZZ V, M^2
-    const Fq r2 = cmul_lazy(qd_sel(k == 3, M, p), qd_sel(k == 3, M, V));
+    const Fq r2 = fe_mul_lazy<FqCfg>(qd_sel(k == 3, M, p), qd_sel(k == 3, M, V));
     const Fq mm = qd_shfl(r2, 3), W = qd_shfl(r2, 1);
     const Fq s2 = fe_add_lazy<FqCfg>(r2, r2);
     const Fq x3 = fe_sub_lazy<FqCfg>(mm, s2);
     const Fq t = fe_sub_lazy<FqCfg>(fe_add_lazy<FqCfg>(s2, r2), mm);  // S - X3
     // M (S - X3), Y W, -, ZZZ W
-    const Fq r3 = cmul_lazy(qd_sel(k == 0, M, p), qd_sel(k == 0, t, W));
+    const Fq r3 = fe_mul_lazy<FqCfg>(qd_sel(k == 0, M, p), qd_sel(k == 0, t, W));
     const Fq y3 = fe_sub_lazy<FqCfg>(qd_shfl(r3, 0), r3);
     return qd_sel(k < 2, qd_sel(k == 0, x3, y3), qd_sel(k == 2, r2, r3));
 }
