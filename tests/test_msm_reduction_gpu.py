@@ -42,3 +42,35 @@ def test_msm_batch_mixed_widths(O, gpu):
     for i, n in enumerate(ns):
         exp = O.msm_known_dlog(d[:n], cols[i][:n]) if n else np.zeros((1, 8), np.uint64)
         assert (O.g1_jac_to_aff(got[i].reshape(1, 12)) == exp).all(), i
+
+
+# the drop-in msm() lays its plan out in the caller's two buffers: scalars split
+# by the endomorphism where the images fit too, whole scalars where not, and a
+# refusal where neither does
+@pytest.mark.parametrize("windows", [20, 30, 44, 54, 64])
+@pytest.mark.parametrize("bits", [3, 5, 7, 10])
+def test_dropin_msm_region_sizes(O, gpu, windows, bits):
+    H, L = gpu.host, gpu.load_library()
+    n, guard = 1000, 4096
+    d = O.rand_fr(n, 91)
+    bases, s = H.to_device(O.g1_gen_bases(d)), O.rand_fr(n, 92)
+    exp = O.msm_known_dlog(d, s)
+    sd = H.to_device(s)
+    for workers in (0, 64, 1024):
+        region = ((windows << bits) + 2 * workers) * 96
+        words = 3 * n * windows * 4
+        res = torch.full((region + guard,), 7, dtype=torch.uint8, device="cuda")
+        srt = torch.full((words + guard,), 7, dtype=torch.uint8, device="cuda")
+        dummy = torch.zeros(64, dtype=torch.int32, device="cuda")
+        p = dummy.data_ptr()
+        st = H.stream_handle()
+        err = L.msm(res.data_ptr(), bases.data_ptr(), sd.data_ptr(), p, p, p, p, srt.data_ptr(), p, n, windows, bits,
+                    64, workers, words, 1, st)
+        assert err in (0, 1)
+        if err == 0:
+            regions = H.ptr_array([res])
+            assert L.batch_msm_collect(p, p, p, p, regions.data_ptr(), workers, windows, bits, 1, st) == 0
+            torch.cuda.synchronize()
+            got = res[:96].cpu().numpy().view(np.uint64)
+            assert (O.g1_jac_to_aff(got.reshape(1, 12)) == exp).all(), workers
+        assert (res[region:] == 7).all() and (srt[words:] == 7).all()
