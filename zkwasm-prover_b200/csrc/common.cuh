@@ -38,6 +38,61 @@ __device__ __forceinline__ void st_elem(Fe<C>* p, const Fe<C>& v) {
     q[1] = make_uint4(v.v[4], v.v[5], v.v[6], v.v[7]);
 }
 
+// fe_inv by a warp, for a chain that waits on one inverse: all lanes call it
+// with the same element and get its inverse.  The four long rows f, g, d, e go to
+// the four lanes of a quad, which apply the matrix side by side (every quad the
+// same), where one thread applies them one after the other: 30400 clocks
+// against 38400.
+template <class C>
+__device__ __forceinline__ Fe<C> fe_inv_warp(const Fe<C>& a) {
+    if (fe_is_zero<C>(a)) return a;  // (uniform)
+    const int k = threadIdx.x & 3;   // row f, g, d or e
+    uint32_t mw[8];
+    int32_t m[9];
+#pragma unroll
+    for (int j = 0; j < 8; j++) mw[j] = C::M(j);
+    Inv30 x;
+#pragma unroll
+    for (int i = 0; i < 9; i++) {
+        m[i] = inv_limb(mw, i);
+        const int32_t g = inv_limb(a.v, i);
+        x.v[i] = k == 0 ? m[i] : k == 1 ? g : (k == 3 && i == 0) ? 1 : 0;
+    }
+    int32_t delta2 = 1;
+#pragma unroll 1
+    for (int round = 0; round < 20; round++) {
+        const uint32_t low = (uint32_t)x.v[0] | ((uint32_t)x.v[1] << 30);
+        const InvMat t = inv_steps(delta2, __shfl_sync(0xffffffffu, low, 0, 4), __shfl_sync(0xffffffffu, low, 1, 4));
+        Inv30 y;
+#pragma unroll
+        for (int i = 0; i < 9; i++) y.v[i] = __shfl_xor_sync(0xffffffffu, x.v[i], 1);
+        // own row and partner: u f + v g, r g + q f, and the same of d, e mod m
+        const int32_t own = (k & 1) ? t.r : t.u, other = (k & 1) ? t.q : t.v;
+        const int64_t M30 = (1 << 30) - 1;
+        int64_t c = (int64_t)own * x.v[0] + (int64_t)other * y.v[0];
+        const int32_t q = k >= 2 ? (int32_t)(((uint32_t)c * C::INV) & (uint32_t)M30) : 0;
+        c += (int64_t)q * m[0];
+        c >>= 30;
+        int32_t nz = 0;
+#pragma unroll
+        for (int i = 1; i < 9; i++) {
+            c += (int64_t)own * x.v[i] + (int64_t)other * y.v[i];
+            c += (int64_t)q * m[i];
+            x.v[i - 1] = (int32_t)(c & M30);
+            nz |= x.v[i - 1];
+            c >>= 30;
+        }
+        x.v[8] = (int32_t)c;
+        nz |= x.v[8];
+        if (!__shfl_sync(0xffffffffu, nz, 1, 4)) break;  // g = 0
+    }
+    const int32_t sign = __shfl_sync(0xffffffffu, x.v[8], 0, 4) < 0 ? -1 : 1;
+    Inv30 d;
+#pragma unroll
+    for (int i = 0; i < 9; i++) d.v[i] = __shfl_sync(0xffffffffu, x.v[i], 2, 4);
+    return inv_finish<C>(d, sign);
+}
+
 // Shared-memory tiles hold 32-byte elements as two 16-byte halves.  Element
 // p, half h lives at 16-byte slot 2 * (p ^ ((p >> 3) & 3)) + (h ^ (((p >> 2) ^
 // (p >> 5)) & 1)): a bijection on each tile that gives the eight threads of a

@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(ST) batch_prod_kernel(Src src, uint32_t n, Fr*
 // K = 8 three blocks fit an SM.  The tree takes 36 products of whole warps a
 // block, where exclusive prefixes and suffixes of the chunk products by two
 // block scans took 176.  Bound by the chain of tree and inversion while it
-// waits (2^15 elements: 114 -> 41 us with K = 2; 2^20: 218 -> 157 us).
+// waits (2^15 elements: 114 -> 30 us with K = 2; 2^20: 218 -> 116 us).
 template <int K>
 static constexpr size_t batch_inv_smem() {
     return (size_t)(K + 1) * ST * sizeof(Fr);
@@ -152,8 +152,10 @@ __global__ void __launch_bounds__(ST, 3) batch_inv_kernel(Src src, Dst dst, uint
     const size_t base = (size_t)blockIdx.x * (ST * K);
     const int t = threadIdx.x;
     const Fr one = fe_one<FrCfg>();
+    // (rolled loops: unrolled, the products are 80 KB of code and the warps wait
+    // for instructions)
     Fr run = one;
-#pragma unroll
+#pragma unroll 1
     for (int k = 0; k < K; k++) {
         const size_t i = base + t + (size_t)ST * k;
         Fr a = one;
@@ -180,33 +182,32 @@ __global__ void __launch_bounds__(ST, 3) batch_inv_kernel(Src src, Dst dst, uint
             if (t < h) node[h + t] = fe_mul<FrCfg>(node[2 * (h + t)], node[2 * (h + t) + 1]);
             __syncwarp();
         }
-        if (t == 0) node[1] = inv_tots ? ld_elem<FrCfg>(inv_tots + blockIdx.x) : fe_inv<FrCfg>(node[1]);
+        const Fr inv = inv_tots ? ld_elem<FrCfg>(inv_tots + blockIdx.x) : fe_inv_warp<FrCfg>(node[1]);
         __syncwarp();
-        // down: the inverses of a node's children
+        if (t == 0) node[1] = inv;
+        __syncwarp();
+        // down: a child's inverse is its parent's times its sibling, a lane a child
 #pragma unroll 1
         for (int h = 1; h <= 16; h <<= 1) {
-            if (t < h) {
-                Fr* c = node + 2 * (h + t);
-                const Fr inv = node[h + t], l = c[0], r = c[1];
-                c[0] = fe_mul<FrCfg>(inv, r);
-                c[1] = fe_mul<FrCfg>(inv, l);
-            }
+            Fr v;
+            if (t < 2 * h) v = fe_mul<FrCfg>(node[h + (t >> 1)], node[(2 * h + t) ^ 1]);
+            __syncwarp();
+            if (t < 2 * h) node[2 * h + t] = v;
             __syncwarp();
         }
     }
     __syncthreads();
 #pragma unroll 1
     for (int h = 32; h < ST; h <<= 1) {
-        if (t < h) {
-            Fr* c = h == ST / 2 ? leaf + 2 * t : node + 2 * (h + t);
-            const Fr inv = node[h + t], l = c[0], r = c[1];
-            c[0] = fe_mul<FrCfg>(inv, r);
-            c[1] = fe_mul<FrCfg>(inv, l);
-        }
+        Fr* c = h == ST / 2 ? leaf : node + 2 * h;
+        Fr v;
+        if (t < 2 * h) v = fe_mul<FrCfg>(node[h + (t >> 1)], c[t ^ 1]);
+        __syncthreads();
+        if (t < 2 * h) c[t] = v;
         __syncthreads();
     }
     Fr cur = leaf[t];
-#pragma unroll
+#pragma unroll 1
     for (int k = K - 1; k >= 0; k--) {
         const size_t i = base + t + (size_t)ST * k;
         Fr a = one;
