@@ -268,7 +268,9 @@ cudaError_t zkp_ntt_batch(void *buf, void *tmp, const void *omegas, const void *
                           size_t col_stride, int *result_in_tmp, cudaStream_t stream);
 
 /* The library's pass split for a transform of 2^log_n points: writes the
- * radices (log2, at most 4) and returns their count (0 if unsupported). */
+ * radices (log2, at most 4) and returns their count (0 if unsupported).
+ * Columns that hold up to 2^16 points in all run two even passes where it has
+ * two. */
 int zkp_ntt_default_plan(int log_n, int *radices);
 
 /* zkp_ntt_batch with the pass split given (host array of npasses radices,

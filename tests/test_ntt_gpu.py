@@ -96,6 +96,20 @@ def test_ntt_batch_columns(O, gpu, log_n, ncols):
         assert (got[c * n:(c + 1) * n] == O.ntt(a[c * n:(c + 1) * n], log_n)).all()
 
 
+@pytest.mark.parametrize("log_n,ncols", [(9, 2), (10, 1), (11, 4), (12, 16)])
+def test_one_pass_transforms_leave_tmp_alone(O, gpu, log_n, ncols):
+    """Where one pass does, tmp may be any buffer: nothing is written there."""
+    H = gpu.host
+    n = 1 << log_n
+    a, b = O.rand_fr(n * ncols, 900 + log_n), O.rand_fr(n * ncols, 950 + log_n)
+    tw = H.generate_omega_buffers(_omega_mont(O, log_n), log_n)
+    buf, tmp = H.to_device(a), H.to_device(b)
+    out = H.ntt_batch(buf, tmp, tw, log_n, ncols)
+    torch.cuda.synchronize()
+    assert out is buf and (H.to_host(tmp) == b).all()
+    assert (H.to_host(out)[:n] == O.ntt(a[:n], log_n)).all()
+
+
 # on both sides of the size up to which passes take two elements a thread, and
 # the smallest sizes of each radix there
 @pytest.mark.parametrize("log_n,ncols", [(7, 1), (8, 3), (9, 5), (10, 64), (10, 65), (11, 1), (12, 16), (12, 17),

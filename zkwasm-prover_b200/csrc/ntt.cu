@@ -893,9 +893,9 @@ cudaError_t ntt_run(Fr* buf, Fr* tmp, const Fr* tw, const Fr* scale, int log_n, 
                     size_t col_stride, bool* result_in_tmp, cudaStream_t s) {
     int rad[4];
     const int np = ntt_plan(log_n, rad);
-    if (log_n >= 10 && ntt_is_short(log_n, ncols) && (np == 2 || (np == 1 && tmp && tmp != buf))) {
-        // two even passes on as many SMs as the columns fill, also where one CTA
-        // could hold a column (the result is in buf either way)
+    if (np == 2 && ntt_is_short(log_n, ncols)) {
+        // two even passes on as many SMs as the columns fill (the result is in buf
+        // either way).  Transforms of one pass keep it: tmp is not theirs to write.
         rad[0] = (log_n + 1) / 2;
         rad[1] = log_n / 2;
         return ntt_run_plan(buf, tmp, tw, scale, log_n, ncols, col_stride, rad, 2, result_in_tmp, s);
