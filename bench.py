@@ -199,7 +199,7 @@ class ExtendPhase:
         return [c * half, c * (half + n), c * E * (half + n), c * E * half]
 
     def launches_per_step(self):
-        return (self.C // self.chunk) * (3 if self.fused() else 4)
+        return (self.C // self.chunk) * 4
 
     def run_chunk(self, c0, events=None, stream=None, lag=None, coeff=None):
         n, E = self.n, self.E
@@ -1082,9 +1082,9 @@ def run_ours(args):
             "graph": {"ms_per_step": round(graph_ms, 3),
                       "value": round(total_bytes / (graph_ms / 1e3) / 1e9, 3), "unit": "GB/s",
                       "launches_per_step": 1},
-            # kernels per chunk: inverse pass 1, the fused stage and coset
-            # pass 2 (four separate passes without the fused stage)
-            "gpu_launches": launches * (3 if ph.fused() else 4),
+            # kernels per chunk: inverse pass 1, the cosets' factors, the fused
+            # stage and coset pass 2 (four separate passes without it)
+            "gpu_launches": launches * 4,
             "roofline": {
                 "bound": "hbm", "achieved": round(achieved, 2), "peak": peak_hbm, "unit": "GB/s",
                 "frac": round(achieved / peak_hbm, 4), "traffic": traffic,
@@ -1565,10 +1565,10 @@ def run_pipeline(args):
 
 
 # kernels each library entry point launches at the proof's sizes (2^22, the
-# batched MSM pipeline over a table), counted from the ncu launch list of one
-# proof (1089 launches of this library's kernels); entry points not listed
-# launch one kernel
-KERNELS_PER_CALL = {"zkp_msm_batch_table": 14, "zkp_ntt_batch_twisted": 2, "zkp_ntt_batch": 2, "ntt": 2,
+# batched MSM pipeline over a table), counted from ncu launch lists; entry
+# points not listed launch one kernel.  A coset transform launches a third
+# kernel (its first pass's factors) that is left out here.
+KERNELS_PER_CALL = {"zkp_msm_batch_table": 15, "zkp_ntt_batch_twisted": 2, "zkp_ntt_batch": 2, "ntt": 2,
                     "calc_m": 2, "prepare_table_lookup": 1, "logup_sum_input_inv": 1, "eval_logup_z_compose": 6,
                     "zkp_permutation_z": 4, "zkp_shuffle_z": 4, "zkp_powers": 2, "zkp_poly_divide_linear": 9,
                     "zkp_poly_eval_batch": 2}
