@@ -1566,8 +1566,7 @@ def run_pipeline(args):
 
 # kernels each library entry point launches at the proof's sizes (2^22, the
 # batched MSM pipeline over a table), counted from ncu launch lists; entry
-# points not listed launch one kernel.  A coset transform launches a third
-# kernel (its first pass's factors) that is left out here.
+# points not listed launch one kernel
 KERNELS_PER_CALL = {"zkp_msm_batch_table": 15, "zkp_ntt_batch_twisted": 2, "zkp_ntt_batch": 2, "ntt": 2,
                     "calc_m": 2, "prepare_table_lookup": 1, "logup_sum_input_inv": 1, "eval_logup_z_compose": 6,
                     "zkp_permutation_z": 4, "zkp_shuffle_z": 4, "zkp_powers": 2, "zkp_poly_divide_linear": 9,

@@ -387,9 +387,9 @@ cudaError_t zkp_shuffle_z(void *z, const void *inputs, const void *tables, const
  * ------------------------------------------------------------------ */
 
 /* NTT of ncols columns from `in` (stride in_stride) into `out` (stride
- * out_stride, out != in): out_c = NTT(in_c[k] * in_mul[k]) (in_mul may be
- * NULL), every output times *scale when scale is non-NULL.  With in_mul[k] =
- * (zeta w_N^j)^k it gives coset j of the extended domain zeta <w_N>
+ * out_stride, out != in): out_c = NTT(in_c[k] * in_mul[k]) for any n factors
+ * in_mul (NULL: none), every output times *scale when scale is non-NULL.  With
+ * in_mul[k] = (zeta w_N^j)^k it gives coset j of the extended domain zeta <w_N>
  * (N = E n) from coefficients.  tmp: n * ncols elements (unused for one-pass
  * sizes).  pairs != 0: omegas, in_mul and scale hold (w, w') known-factor
  * pairs (zkp_shoup_pairs), 2 elements an entry. */

@@ -109,8 +109,39 @@ def test_cosets_and_combine(O, gpu, P, ext_bits, pairs):
     assert (_h(out) == exp).all()
 
 
-# two passes with every remainder of the in-block radix (7+6, 6+8, 9+9, 11+10)
-# and three (11+6+6): the coset's factors come from the first pass's own table
+# the factors of zkp_ntt_batch_twisted are any, not only the powers of a shift:
+# short and radix-8 passes (7+6, 9+9, 11+6+6), both table layouts
+@pytest.mark.parametrize("log_n,cols", [(12, 2), (13, 2), (13, 64), (18, 2), (23, 1)])
+@pytest.mark.parametrize("pairs", [False, True])
+@pytest.mark.parametrize("factors", ["random", "scaled"])
+def test_twisted_transform_takes_any_factors(O, gpu, P, log_n, cols, pairs, factors):
+    L = gpu.load_library()
+    n = 1 << log_n
+    tab = P.Tables(log_n)
+    if factors == "random":
+        mul = O.rand_fr(n, 230 + log_n)
+    else:  # c s^k, whose first entry is not one
+        c, s = O.fr_ints(O.rand_fr(2, 231))
+        mul = O.mul(_h(P.powers(1, s, n)), O.fr_vec([c]))
+    tw, tm = tab.tw, RC.Dev().put(mul)
+    if pairs:
+        tw, tp = (torch.empty((2 * n, 4), dtype=torch.int64, device="cuda") for _ in range(2))
+        assert L.zkp_shoup_pairs(tw.data_ptr(), tab.tw.data_ptr(), n, 0) == 0
+        assert L.zkp_shoup_pairs(tp.data_ptr(), tm.data_ptr(), n, 0) == 0
+        tm = tp
+    x = O.rand_fr(cols * n, 232)
+    src = RC.Dev().put(x)
+    tmp, out = (torch.empty((cols * n, 4), dtype=torch.int64, device="cuda") for _ in range(2))
+    assert L.zkp_ntt_batch_twisted(out.data_ptr(), src.data_ptr(), tmp.data_ptr(), tw.data_ptr(), tm.data_ptr(), 0,
+                                   log_n, cols, n, n, int(pairs), 0) == 0
+    got = _h(out)
+    for c in {0, cols // 2, cols - 1}:
+        exp = O.ntt(O.mul(x[c * n:(c + 1) * n], mul), log_n)
+        assert (got[c * n:(c + 1) * n] == exp).all(), c
+
+
+# powers of a shift in two passes with every remainder of the in-block radix
+# (7+6, 6+8, 9+9, 11+10) and three (11+6+6), strides wider than a column
 @pytest.mark.parametrize("log_n", [13, 14, 16, 18, 21, 23])
 @pytest.mark.parametrize("pairs", [False, True])
 def test_coset_transform_of_several_passes(O, gpu, P, log_n, pairs):

@@ -23,7 +23,6 @@ struct NttPassArgs {
     size_t src_zs, dst_zs;  // per-sub-transform strides (blockIdx.z), elements
     size_t in_mul_zs;
     int pairs;           // tw, in_mul and scale hold (w, w') pairs (two elements an entry)
-    const Fr* ctab;      // first pass of a coset transform: its factors (ntt_coset_table), with in_mul
 };
 
 cudaError_t ntt_pass(const NttPassArgs& a, int log_r, unsigned ny, unsigned nz, cudaStream_t s);

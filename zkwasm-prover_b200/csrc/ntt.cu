@@ -17,14 +17,16 @@
 //   - a factor common to all inputs (the scale n^-1) costs one product per
 //     eight elements: it goes into the eight factors of an item's first
 //     sub-stage, where input 0 otherwise has none;
-//   - a coset shift s (X[j] = sum_k x_k s^k w^{jk}) only changes factors that
-//     are multiplied by anyway: see ntt_coset_table_kernel.
+//   - in the fused extension a coset shift s (X[j] = sum_k x_k s^k w^{jk}) only
+//     changes factors that are multiplied by anyway: see ntt_coset_table_kernel.
 //
 // Twiddles come from the natural table w^i (i < n) that expand_omega_buffer
 // builds; a sub-stage twiddle w_R^e is entry e * (n/R).
 //
 // The same pass kernel serves the coset extension: an optional per-input
-// multiplier table (the coset twist s^k, applied on load in the first pass),
+// multiplier table (the coset twist s^k or any other factors, applied in the
+// first pass, whose first sub-stage has no twiddles: the products an element
+// are the same as with the shift in the sub-stages' factors),
 // an optional output scale (n^-1 for the inverse transform) and an output
 // index map pos -> (pos << out_shift) + z * out_off_z that interleaves the
 // 2^e sub-transforms of an extended domain.
@@ -222,8 +224,8 @@ __device__ __forceinline__ void dft4_dif(Fr& v0, Fr& v1, Fr& v2, Fr& v3, const t
 }
 
 // Where the factors of an item's sub-stages come from: the table of w_n at
-// (i J_full) n / (P R_s) for item index J_full = J + P Jl, or ctab, the table
-// of a coset's first pass (ntt_coset_table_kernel).
+// (i J_full) n / (P R_s) for item index J_full = J + P Jl, or ctab, the fused
+// extension's table of a coset's first pass (ntt_coset_table_kernel).
 struct StageTw {
     const Fr* tw;
     const Fr* ctab;
@@ -397,24 +399,18 @@ ntt_pass_kernel(NttPassArgs a) {
     const Fr* src = a.src + by * a.src_ys + blockIdx.z * a.src_zs;
     Fr* dst = a.dst + by * a.dst_ys + blockIdx.z * a.dst_zs;
 
-    // factors of the first sub-stage's eight inputs, one set an item, where all
-    // eight are multiplied: a scale (times the item's twiddles), or the first
-    // pass of a coset transform with its own table
+    // factors of the first sub-stage's eight inputs, one set an item, where a
+    // scale multiplies all eight (times the item's twiddles)
     __shared__ Fr kst[G * 8 * TW::EW];
     __shared__ DftK<TW> dk;
-    const bool kst_used = a.ctab || (a.scale && !a.in_mul);
+    const bool kst_used = a.scale && !a.in_mul;
     dk.init(a.tw, a.log_n);
     if (kst_used) {
         for (int k = tid; k < G * 8; k += T) {
             const uint32_t qk = q0 + k / 8, i = k % 8;
-            typename TW::K f;
-            if (a.ctab) {
-                f = TW::ld(a.in_mul, (size_t)qk + ((size_t)i << (a.log_n - 3)));
-            } else {
-                f = TW::ld(a.scale, 0);
-                const uint32_t J = qk & ((1u << a.log_p) - 1);
-                if (i * J) f = TW::prod(TW::ld(a.tw, (size_t)(i * J) << (a.log_n - a.log_p - 3)), f);
-            }
+            typename TW::K f = TW::ld(a.scale, 0);
+            const uint32_t J = qk & ((1u << a.log_p) - 1);
+            if (i * J) f = TW::prod(TW::ld(a.tw, (size_t)(i * J) << (a.log_n - a.log_p - 3)), f);
             TW::put(kst + k * TW::EW, f);
         }
     }
@@ -433,7 +429,7 @@ ntt_pass_kernel(NttPassArgs a) {
     const Fr* in_mul = a.in_mul ? TW::off(a.in_mul, blockIdx.z * a.in_mul_zs) : nullptr;
     StageTw st;
     st.tw = a.tw;
-    st.ctab = a.ctab;
+    st.ctab = nullptr;
     st.log_n = a.log_n;
     st.log_p = a.log_p;
     st.J = q & ((1u << a.log_p) - 1);
@@ -443,9 +439,20 @@ ntt_pass_kernel(NttPassArgs a) {
     if (kst_used) {
         stage8_scale<TW>(v, kst + g * 8 * TW::EW);
     } else if (in_mul) {
+        // any factors, one an element (the first pass has no twiddles here)
+        const size_t m0 = (size_t)q + ((size_t)lt << log_items), ms = (size_t)TR << log_items;
+        if constexpr (TW::EW == 2) {
 #pragma unroll
-        for (int i = 0; i < 8; i++)
-            v[i] = TW::mul(v[i], TW::ld(in_mul, (size_t)q + ((size_t)(lt + TR * i) << log_items)));
+            for (int i = 0; i < 8; i++) v[i] = TW::mul(v[i], TW::ld(in_mul, m0 + i * ms));
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) {
+                const Fr2 m = TW::mul2(v[i], TW::ld(in_mul, m0 + i * ms), v[i + 1],
+                                       TW::ld(in_mul, m0 + (i + 1) * ms));
+                v[i] = m.a;
+                v[i + 1] = m.b;
+            }
+        }
         if (a.scale) {
 #pragma unroll
             for (int i = 0; i < 8; i++) v[i] = TW::mul(v[i], TW::ld(a.scale, 0));
@@ -608,11 +615,9 @@ static cudaError_t fused_dispatch(const FusedExtendArgs& a, int log_r, unsigned 
 // DFT runs over x_(q + (n/R) i) s^((n/R) i) (s^q goes into its first
 // sub-stage), so a sub-stage of radix r after P_s multiplies input i of local
 // item Jl by s^(i n/(P_s r)) w_(P_s r)^(i Jl): the same factors for every q and
-// column, at entry r (P_s + Jl) + i, 2 R entries a coset.  s^k is entry
-// k step of pw (k step < n powers of s at step 1, or the R powers of s^(n/R)
-// with the exponents counted in n/R: pw_shift = log2(n/R)).
-// Made once per call into a buffer the first pass does not write, it takes
-// the place of one product an element (the twist of every input).
+// column, at entry r (P_s + Jl) + i, 2 R entries a coset.  pw holds the R powers
+// of s^(n/R), so s^k is its entry k >> pw_shift, pw_shift = log2(n/R).
+// Made once per call into a buffer the first pass does not write.
 template <class TW>
 __global__ void ntt_coset_table_kernel(Fr* ctab, const Fr* pw, size_t pw_zs, int pw_shift, const Fr* tw, int log_n,
                                        int log_r) {

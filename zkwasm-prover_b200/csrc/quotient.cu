@@ -390,13 +390,6 @@ cudaError_t zkp_ntt_batch_twisted(void* out, const void* in, void* tmp, const vo
         a.src_ys = src_stride;
         a.dst_ys = to_out ? out_stride : n;
         a.pairs = pairs ? 1 : 0;
-        if (p == 0 && in_mul && np > 1 && (pairs || !ntt_is_short(log_n, ncols))) {
-            // the twist goes into the first pass's factors, made in the buffer
-            // this pass does not write (n >= 64 R elements)
-            Fr* ctab = to_out ? reinterpret_cast<Fr*>(tmp) : reinterpret_cast<Fr*>(out);
-            ZK_CHECK(ntt_coset_table(ctab, a.in_mul, 0, 0, a.tw, log_n, rad[0], 1, a.pairs, stream));
-            a.ctab = ctab;
-        }
         ZK_CHECK(ntt_pass(a, rad[p], ncols, 1, stream));
         src = dst;
         src_stride = a.dst_ys;
