@@ -236,3 +236,104 @@ def test_eval_h_fused_matches_restatement(O, gpu, P):
         t = O.shuffle_eval_h_v2(t, [q[1], q[3]], [q[2], q[4]], O.fr_vec(sbetas), q[0], l0, ll, la, yv, rs)
     t = O.mul(t, scale)
     assert (_h(h) == t).all()
+
+
+def _eval_h_both(O, gpu, P, n, rs, terms, chunks, chunk_len, lookups, groups, scaled=True):
+    """zkp_eval_h_fused and the oracle's chain over random columns: gate terms
+    as lists of rotations, `chunks` permutation chunks, `lookups`, and one
+    shuffle for each of `groups` (input, table) pair counts."""
+    L, R = gpu.load_library(), O.R_MOD
+    rnd = iter(range(5000, 100_000))
+    pool = [O.rand_fr(n, next(rnd)) for _ in range(24)]  # columns, reused in turn
+    at = iter(range(10 ** 6))
+    col = lambda: pool[next(at) % len(pool)]  # noqa: E731
+    y, beta, gamma = [O.fr_ints(O.rand_fr(1, s))[0] for s in (21, 22, 23)]
+    yv, bv, gv = O.fr_vec([y]), O.fr_vec([beta]), O.fr_vec([gamma])
+    d = RC.Dev()
+    dev = [d.put(c) for c in pool]
+    at_dev = lambda c: next(t for p, t in zip(pool, dev) if p is c)  # noqa: E731
+    l0, ll, la, X = pool[20], pool[21], pool[22], pool[23]
+    gates = [(O.rand_fr(1, next(rnd)), [(col(), r) for r in rots]) for rots in terms]
+    v, rots = [], []
+    for c_, fs in gates:
+        v.append(d.put(c_))
+        v += [at_dev(cc) for cc, _ in fs]
+        rots += [r for _, r in fs]
+        v.append(None)
+    m = max(0, chunks * chunk_len - 1)  # the last chunk is a column short
+    pc, ps, pz = [col() for _ in range(m)], [col() for _ in range(m)], [col() for _ in range(chunks)]
+    db = [beta * pow(P.DELTA, c, R) % R for c in range(m)]
+    lk = [[col() for _ in range(4)] for _ in range(lookups)]
+    sh = [[col() for _ in range(1 + 2 * g)] for g in groups]
+    sbetas = [pow(beta, i + 1, R) for i in range(max(groups, default=1))]
+    last = -3
+    a = P._EvalHArgs()
+    a.n, a.rot_scale = n, rs
+    keep = [d.put(yv), d.put(bv), d.put(gv)]
+    a.y, a.beta, a.gamma = [t.data_ptr() for t in keep]
+    a.l0, a.l_last, a.l_active, a.x = [at_dev(c).data_ptr() for c in (l0, ll, la, X)]
+
+    def put(name, t):
+        keep.append(t)
+        setattr(a, name, t.data_ptr())
+
+    if gates:
+        put("gate_terms", d.ptrs(v))
+        put("gate_rots", d.i32(rots or [0]))
+    if chunks:
+        put("perm_z", d.ptrs([at_dev(c) for c in pz]))
+        put("perm_cols", d.ptrs([at_dev(c) for c in pc]))
+        put("perm_sigmas", d.ptrs([at_dev(c) for c in ps]))
+        put("perm_dbeta", d.put(O.fr_vec(db)))
+    if lookups:
+        put("lookup_cols", d.ptrs([at_dev(c) for q in lk for c in q]))
+    if groups:
+        put("shuffle_cols", d.ptrs([at_dev(c) for q in sh for c in q]))
+        put("shuffle_group_len", d.i32(list(groups)))
+        put("shuffle_betas", d.put(O.fr_vec(sbetas)))
+    scale = O.rand_fr(1, 24)
+    if scaled:
+        put("scale", d.put(scale))
+    a.gate_terms_n = len(v)
+    a.perm_chunks, a.perm_chunk_len, a.perm_cols_n, a.perm_last_rot = chunks, chunk_len, m, last
+    a.lookups, a.shuffles = lookups, len(groups)
+    h = torch.empty((n, 4), dtype=torch.int64, device="cuda")
+    assert L.zkp_eval_h_fused(h.data_ptr(), ctypes.byref(a), 0) == 0
+    t = O.field_op_batch_mul_sum(O.zeros(n), [(c_, [(cc, r * rs) for cc, r in fs]) for c_, fs in gates], n)
+    if chunks:
+        t = O.permutation_eval_h_p1(t, pz[0], pz[-1], l0, ll, yv)
+        t = O.permutation_eval_h_p2(t, pz, l0, ll, yv, last * rs)
+    for j in range(chunks):
+        Lp, Rp = O._rot(pz[j], rs), pz[j]
+        for c in range(chunk_len * j, min(m, chunk_len * (j + 1))):
+            Lp = O.mul(Lp, O.add(O.add(pc[c], O.mul(ps[c], bv)), gv))
+            Rp = O.mul(Rp, O.add(O.add(pc[c], O.mul(X, O.fr_vec([db[c]]))), gv))
+        t = O.add(O.mul(t, yv), O.mul(la, O.sub(Lp, Rp)))
+    for q in lk:
+        t = O.logup_eval_h(t, O.add(q[0], bv), O.one(n), O.add(q[1], bv), q[2], q[3], q[3], l0, ll, la, yv, rs)
+    for q in sh:
+        t = O.shuffle_eval_h_v2(t, q[1::2], q[2::2], O.fr_vec(sbetas), q[0], l0, ll, la, yv, rs)
+    if scaled:
+        t = O.mul(t, scale)
+    return _h(h), t
+
+
+# every combination of absent families, one and several shuffles, and both block
+# sizes (128 threads up to 151552 rows, 256 above)
+@pytest.mark.parametrize("n", [1, 64, 1 << 10, 1 << 18])
+@pytest.mark.parametrize("gates,chunks,lookups,groups", [
+    (3, 0, 0, ()), (0, 3, 0, ()), (0, 0, 2, ()), (0, 0, 0, (2,)), (2, 1, 0, ()), (2, 2, 0, (1, 3)),
+    (2, 0, 3, (2, 1)), (1, 3, 2, (1, 2, 3))])
+def test_eval_h_fused_families(O, gpu, P, n, gates, chunks, lookups, groups):
+    terms = [[0], [1, -1, 2], [-2, 0]][:gates]
+    got, exp = _eval_h_both(O, gpu, P, n, 1 if n < 1 << 10 else 2, terms, chunks, 2, lookups, groups, n != 64)
+    assert (got == exp).all()
+
+
+# gate lists longer than the coefficients staged per block (entries below 256):
+# terms that start on either side of the line, coefficients without a column
+@pytest.mark.parametrize("tail", [[0, 0, 0, 2, 1], [0, 2, 1, 0, 3], [1, 1, 1, 0]])
+def test_eval_h_fused_long_gate_lists(O, gpu, P, tail):
+    terms = [[t % 3 - 1] for t in range(84)] + [[i - 1 for i in range(k)] for k in tail]  # the tail starts at 252
+    got, exp = _eval_h_both(O, gpu, P, 1 << 10, 1, terms, 2, 3, 1, (1,))
+    assert (got == exp).all()

@@ -96,9 +96,17 @@ struct EvalHView {
 // coefficients, are staged per block as known factors
 static constexpr int EVAL_H_MAX_PERM = 256;
 static constexpr int EVAL_H_MAX_TERMS = 128;
-// threads a block: four blocks of 128 an SM share the rows out more evenly than
-// two of 256 (2^17 rows: 1.28 against 1.44 ms)
-static constexpr int EH_TB = 128;
+// Threads a block: 256, two blocks an SM, or 128 and four blocks up to
+// EH_SHORT_ROWS rows.  There an SM has at most four blocks of 256, and blocks of
+// 128 share the rows out more evenly (17 gates, 60 permutation columns, 24
+// lookups, 4 shuffles: 2^14 rows 0.37 against 0.45 ms, 2^17 1.25 against 1.33).
+// Above, blocks of 256 are faster (2^18 rows 2.32 against 2.46 ms, 2^20 9.1
+// against 9.8, 2^22 35.5 against 44.4; 46 columns in all, 2^22 rows: 5.3 against
+// 7.1): the longer four blocks run, the further apart they are in the kernel's
+// code, and its warps wait for instructions (46 columns, 2^20 rows: 3.2 cycles
+// an issue against 0.6).
+static constexpr int EH_TB = 256;
+static constexpr uint32_t EH_SHORT_ROWS = 4 * 148 * EH_TB;
 
 // The factors fixed for a launch, in known-factor form: beta and the powers
 // of y the sum over constraints needs.
@@ -114,11 +122,12 @@ enum { EH_BETA, EH_Y, EH_Y2, EH_Y3, EH_YG, EH_Y0, EH_YL, EH_FACTORS };
 // both are z, so one accumulator serves both), A the chunk products in y and
 // then the third constraints in y^3.  A lookup costs two products by the known
 // y^3 and two full ones instead of three and five, a chunk link or product one
-// known product instead of one of each.  Bound by the multiply pipe: at 2^17
-// rows of 17 gates, 60 permutation columns, 24 lookups and 4 shuffles
-// 1.25 ms, 1.59 with one accumulator in y for every constraint and without the
-// prefetch of the next column (1.28 without the prefetch alone).
-__global__ void __launch_bounds__(EH_TB, 512 / EH_TB) eval_h_fused_kernel(Fr* h, EvalHView a) {
+// known product instead of one of each.  Bound by the multiply pipe: at 17
+// gates, 60 permutation columns, 24 lookups and 4 shuffles 2^17 rows take
+// 1.25 ms and 2^22 35.5 ms; with one accumulator in y for every constraint and
+// without the prefetch of the next column 1.59 and 44.0 (without the prefetch
+// alone 1.28 and 36.5).
+__global__ void __launch_bounds__(EH_TB, 2) eval_h_fused_kernel(Fr* h, EvalHView a) {
     __shared__ KnownFr s_dbeta[EVAL_H_MAX_PERM];
     __shared__ KnownFr s_coef[EVAL_H_MAX_TERMS];
     __shared__ KnownFr s_k[EH_FACTORS];
@@ -441,7 +450,8 @@ cudaError_t zkp_eval_h_fused(void* h, const zkp_eval_h_args* args, cudaStream_t 
     v.shuffle_group_len = reinterpret_cast<const int*>(g.shuffle_group_len);
     v.shuffle_betas = CFr(g.shuffle_betas);
     v.scale = CFr(g.scale);
-    eval_h_fused_kernel<<<qz_grid(n, EH_TB), EH_TB, 0, stream>>>(reinterpret_cast<Fr*>(h), v);
+    const unsigned tb = n <= EH_SHORT_ROWS ? EH_TB / 2 : EH_TB;
+    eval_h_fused_kernel<<<qz_grid(n, tb), tb, 0, stream>>>(reinterpret_cast<Fr*>(h), v);
     return cudaGetLastError();
 }
 
