@@ -74,3 +74,24 @@ def test_dropin_msm_region_sizes(O, gpu, windows, bits):
             got = res[:96].cpu().numpy().view(np.uint64)
             assert (O.g1_jac_to_aff(got.reshape(1, 12)) == exp).all(), workers
         assert (res[region:] == 7).all() and (srt[words:] == 7).all()
+
+
+# sets and windows without a point: no scalar but zero, and scalars whose one
+# digit lies in the lowest, a middle or the topmost window
+@pytest.mark.parametrize("n", [1, 3, 40])
+@pytest.mark.parametrize("value", [0, 1, 1 << 19, 1 << 64, 1 << 126, (1 << 253) + 1])
+@pytest.mark.parametrize("dense", [False, True])
+def test_msm_empty_windows(O, gpu, n, value, dense):
+    H = gpu.host
+    d = O.rand_fr(n, 171)
+    bases = H.to_device(O.g1_gen_bases(d))
+    s = O.fr_vec([value if dense or i == n // 2 else 0 for i in range(n)])
+    exp = O.msm_known_dlog(d, s)
+    sd = H.to_device(s)
+    table, c = H.msm_table_build(bases, n, 0)
+    outs = [H.msm(bases, sd, n=n), H.msm(bases, sd, n=n, window_bits=13), H.msm_table(table, n, c, sd, n=n)]
+    outs += [H.msm_batch(bases, [sd, sd], [n, n], [4, 11])]
+    torch.cuda.synchronize()
+    for out in outs:
+        for got in H.to_host(out).reshape(-1, 12):
+            assert (O.g1_jac_to_aff(got.reshape(1, 12)) == exp).all()

@@ -140,13 +140,14 @@ __device__ __forceinline__ Xyzz qd_point(const Fq& p) {
 // all compute the same)
 __device__ __forceinline__ Jac coop_horner(const Xyzz* win, int W, int c) {
     Fq acc = fe_zero<FqCfg>();
-    if (W > 0) acc = qd_load(win + W - 1);
-    for (int w = W - 2; w >= 0; w--) {
+    int w = W - 1;
+    if (w >= 0) acc = qd_load(win + w);
+    // small scalars leave the top windows empty
+    while (w > 0 && __all_sync(0xffffffffu, fe_is_zero<FqCfg>(acc))) acc = qd_load(win + --w);
+    while (--w >= 0) {
         const Fq next = qd_load(win + w);
-        // small scalars leave the top windows empty
-        const int dbl = __all_sync(0xffffffffu, fe_is_zero<FqCfg>(acc)) ? 0 : c;
 #pragma unroll 1
-        for (int i = 0; i < dbl; i++) acc = qd_dbl(acc);
+        for (int i = 0; i < c; i++) acc = qd_dbl(acc);
         acc = qd_add(acc, next);
     }
     return xyzz_to_jac(qd_point(acc));
@@ -198,7 +199,10 @@ __device__ __forceinline__ void red_tree(Xyzz* Tp, Xyzz* Sp, uint32_t lg) {
                 p = reinterpret_cast<const Fq*>(dst)[qd_lane()];
                 q = reinterpret_cast<const Fq*>(dst + (1u << (l - 1)))[qd_lane()];
             }
-            p = qd_add(p, q);
+            // skipped where no quad of the warp has two points (an identity's
+            // components are all zero): empty buckets, short and sparse columns
+            const bool zq = fe_is_zero<FqCfg>(q);
+            p = __all_sync(0xffffffffu, zq || fe_is_zero<FqCfg>(p)) ? qd_sel(zq, p, q) : qd_add(p, q);
             if (live) reinterpret_cast<Fq*>(dst)[qd_lane()] = p;
         }
         __syncthreads();
@@ -255,12 +259,20 @@ __device__ __forceinline__ Fq red_horner(const Xyzz* set, uint32_t G, uint32_t s
     const uint32_t H = G > RED_T ? G / RED_T : 1u;
     const Xyzz* v = H > 1 ? set + RED_PLANES * H : set;
     Fq acc = fe_zero<FqCfg>();
-    // the bits of the segment number from the top, seg's doublings, then S
+    // the bits of the segment number from the top, seg's doublings, then S;
+    // leading identities (an empty set has only those) cost nothing
     uint32_t k = 31u - (uint32_t)__clz((int)G), s = seg;
+    bool some = false;
 #pragma unroll 1
     while (s) {
-        if (k > 0 || s > 1) acc = qd_dbl(acc);
-        if (k > 0 || s == 1) acc = qd_add(acc, qd_load(v + k));
+        const bool term = k > 0 || s == 1;
+        if (some) {
+            if (k > 0 || s > 1) acc = qd_dbl(acc);
+            if (term) acc = qd_add(acc, qd_load(v + k));
+        } else if (term) {
+            acc = qd_load(v + k);
+            some = !__all_sync(0xffffffffu, fe_is_zero<FqCfg>(acc));
+        }
         if (k > 0)
             k--;
         else
