@@ -95,3 +95,21 @@ def test_msm_empty_windows(O, gpu, n, value, dense):
     for out in outs:
         for got in H.to_host(out).reshape(-1, 12):
             assert (O.g1_jac_to_aff(got.reshape(1, 12)) == exp).all()
+
+
+# batches whose buckets take segments of 16, of 32 on either side of four blocks
+# an SM, and of 64 (the scratch's limit)
+@pytest.mark.parametrize("count", [12, 24, 48, 60])
+def test_msm_batch_segment_lengths(O, gpu, count):
+    H = gpu.host
+    n, c = 64, 14
+    d = O.rand_fr(n, 151)
+    bases = H.to_device(O.g1_gen_bases(d))
+    cols = [O.rand_fr(n, 160 + i) for i in range(4)]
+    dev = [H.to_device(x) for x in cols]
+    out = H.msm_batch(bases, [dev[i % 4] for i in range(count)], [n] * count, [c] * count)
+    torch.cuda.synchronize()
+    got = O.g1_jac_to_aff(H.to_host(out).reshape(-1, 12))
+    exp = [O.msm_known_dlog(d, x) for x in cols]
+    for i in range(count):
+        assert (got[i] == exp[i % 4][0]).all(), i

@@ -547,12 +547,17 @@ int msm_batch_table_default_window(const uint32_t* n, uint32_t count) {
 // Buckets a reduction segment sums (a power of two) when a launch reduces NB
 // buckets in all, in sets of B: a segment of s buckets costs 2 (s - 1)
 // additions one after the other, a group's tree 14 warp additions whatever s
-// is, so segments are as long as leaves every SM two blocks of 128 segments;
-// and long enough for max_threads segments in all (the scratch they are kept
-// in) and RED_MAX_G a set.
+// is, so short segments double as long as that leaves two blocks of 128
+// segments an SM.  From 32 buckets the tree is a small part and the blocks'
+// number evens out the SMs: those double only while four blocks an SM are left
+// (256 MSMs of 2^14..2^22 points: segments of 1024 497 ms, of 2048 526).  In any
+// case long enough for max_threads segments in all (the scratch they are kept
+// in; one MSM's 32768 are below two blocks an SM) and RED_MAX_G a set.
 uint32_t msm_reduce_segment(uint64_t NB, uint32_t B, uint32_t max_threads) {
     uint32_t s = 1;
-    while (s < B && (NB / s > max_threads || B / s > RED_MAX_G || NB / (2 * (uint64_t)s) >= 2ull * 148 * RED_T)) s *= 2;
+    while (s < B && (NB / s > max_threads || B / s > RED_MAX_G ||
+                     NB / (2 * (uint64_t)s) >= (s < 32 ? 2ull : 4ull) * 148 * RED_T))
+        s *= 2;
     return s;
 }
 
