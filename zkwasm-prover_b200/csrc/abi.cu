@@ -304,7 +304,8 @@ cudaError_t msm(void* res, void* p, void* s, void* indices_buf0, void* indices_b
     const size_t region_bytes = (((size_t)windows << window_bits) + 2 * (size_t)workers) * sizeof(Jac);
     const size_t head = 256;  // res[0] (the result) and the parked note stay clear of the scratch points
     if (region_bytes <= head) return cudaErrorInvalidValue;
-    const int c0 = msm_make_plan(n, 0, false).c;
+    const MsmPlan whole = msm_make_plan(n, 0, false);
+    const int c0 = whole.c;
     int order[40];
     int no = 0;
     order[no++] = c0;
@@ -321,10 +322,21 @@ cudaError_t msm(void* res, void* p, void* s, void* indices_buf0, void* indices_b
     // a point) fit beside the plan, else whole 254-bit scalars: the split halves
     // the windows, so the buckets to reduce and the doublings of the final
     // combination, for one product a base (4 columns of 2^16: 3.17 -> 2.75 ms).
-    // Preferred window first, then (whole scalars) wider and narrower ones until
-    // the plan fits.
+    // Its window is the preferred one, or where that makes more buckets than
+    // whole scalars have (from about 2.2 to 7 million points: 19 bits for 17),
+    // the one of the fewest windows and then the fewest buckets below that:
+    // columns of small or few values fill few buckets and pay for all
+    // (2^22 points at 19 bits: 16-bit scalars 2.61 ms, 1.97 as whole ones).
+    // Whole scalars take the preferred window first, then wider and narrower
+    // ones until the plan fits.
+    MsmPlan split = msm_make_plan(n, 0, true);
+    if (split.NB > whole.NB) {
+        while (split.c > 4 && split.NB > whole.NB) split = msm_make_plan(n, split.c - 1, true);
+        while (split.c > 4 && msm_make_plan(n, split.c - 1, true).W == split.W)
+            split = msm_make_plan(n, split.c - 1, true);
+    }
     for (int i = -1; i < no; i++) {
-        const MsmPlan pl = i < 0 ? msm_make_plan(n, 0, true) : msm_make_plan(n, order[i], false);
+        const MsmPlan pl = i < 0 ? split : msm_make_plan(n, order[i], false);
         MsmScratch sc = {};
         if (msm_layout_arenas(pl, arena, arena_bytes, 2, &sc, 1))
             // the final combination runs in batch_msm_collect, for all MSMs at once
