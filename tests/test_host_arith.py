@@ -196,6 +196,21 @@ def test_xyzz_formulas(O, hc):
     assert O.fq_ints(j[8:])[0] == 0 and O.fq_ints(j[4:8])[0] == 1
 
 
+def test_glv_split_short_scalars(O, hc):
+    """Scalars below 2^96 skip the split's products; the halves stay the same
+    on either side of the line."""
+    ks = [0, 1, 2 ** 32, 2 ** 64 - 1, 2 ** 95, 2 ** 96 - 1, 2 ** 96, 2 ** 96 + 1, 2 ** 97, 2 ** 124, 2 ** 126]
+    k = np.array([[(x >> (64 * j)) & (2 ** 64 - 1) for j in range(4)] for x in ks], np.uint64)
+    m1, m2 = np.empty_like(k), np.empty_like(k)
+    neg = np.empty((len(ks), 2), np.int32)
+    hc.hc_glv_split(_p(k), _p(m1), _p(m2), _p(neg), len(ks))
+    val = lambda r: sum(int(r[j]) << (64 * j) for j in range(4))  # noqa: E731
+    for i, x in enumerate(ks):
+        got = (-val(m1[i]) if neg[i, 0] else val(m1[i]), -val(m2[i]) if neg[i, 1] else val(m2[i]))
+        assert got == O.glv_split(x)
+        assert x >= 2 ** 96 or got == (x, 0)
+
+
 def test_glv_split_matches_restatement(O, hc):
     rng = random.Random(17)
     ks = [0, 1, 2, O.R_MOD - 1, O.R_MOD // 2, O.GLV_LAMBDA, (O.R_MOD - 1) // 3, (1 << 253) - 1]

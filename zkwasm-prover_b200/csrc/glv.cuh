@@ -63,6 +63,14 @@ ZK_HD bool glv_abs(uint32_t* x, int n) {
 // k (canonical, < r) -> magnitudes m1, m2 (< 2^127, 8 limbs, upper four zero)
 // and signs with k = (-1)^neg1 m1 + (-1)^neg2 m2 lambda (mod r)
 ZK_HD void glv_split(const uint32_t k[8], uint32_t m1[8], uint32_t m2[8], bool& neg1, bool& neg2) {
+    if (!(k[3] | k[4] | k[5] | k[6] | k[7])) {  // k g1 < 2^226: c1 = c2 = 0
+        for (int j = 0; j < 8; j++) {
+            m1[j] = k[j];
+            m2[j] = 0;
+        }
+        neg1 = neg2 = false;
+        return;
+    }
     const uint32_t g1[5] = {0x00ff6565u, 0x5398fd03u, 0xa773d2d2u, 0x4ccef014u, 0x00000002u};
     const uint32_t g2[3] = {0xc7e0b3d7u, 0xd91d232eu, 0x00000002u};
     const uint32_t a1[4] = {0x7d4f1128u, 0x8211bbebu, 0xeeb859fcu, 0x6f4d8248u};

@@ -131,7 +131,8 @@ __global__ void msm_count_kernel(const Fr* __restrict__ scalars, uint32_t n, int
 template <bool GLV>
 __global__ void msm_scatter_kernel(const Fr* __restrict__ scalars, uint32_t n, int c, int W, uint32_t kw,
                                    uint32_t pw, uint32_t phi_off, const uint32_t* __restrict__ offset,
-                                   uint32_t* __restrict__ count, uint32_t* __restrict__ entries) {
+                                   uint32_t* __restrict__ count, uint32_t* __restrict__ entries,
+                                   const Aff* __restrict__ bases, Aff* __restrict__ phi) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i - (threadIdx.x & 31) >= n) return;  // whole warps past the end
     const Fr k = i < n ? fe_from_mont<FrCfg>(ldg_elem<FrCfg>(scalars + i)) : fe_zero<FrCfg>();
@@ -141,6 +142,12 @@ __global__ void msm_scatter_kernel(const Fr* __restrict__ scalars, uint32_t n, i
         glv_split(k.v, m1, m2, n1, n2);
         scatter_digits(m1, c, W, kw, i, pw, n1, offset, count, entries);
         scatter_digits(m2, c, W, kw, phi_off + i, pw, n2, offset, count, entries);
+        // the base's image, only where an entry refers to it
+        if (phi && (m2[0] | m2[1] | m2[2] | m2[3])) {
+            const Aff r = glv_phi(ld_aff(bases + i));
+            st_elem<FqCfg>(&phi[i].x, r.x);
+            st_elem<FqCfg>(&phi[i].y, r.y);
+        }
     } else {
         scatter_digits(k.v, c, W, kw, i, pw, false, offset, count, entries);
     }
@@ -788,12 +795,10 @@ cudaError_t msm_run(Jac* out, const Aff* bases, const Fr* scalars, const MsmPlan
     ZK_CHECK(scan_u32(s.count, s.offset, p.NB, s.scan_tmp, st));
     if (p.glv) {
         msm_scatter_kernel<true><<<nblk, tb, 0, st>>>(scalars, p.n, p.c, p.W, kw, pw, phi_off, s.offset, s.count,
-                                                      s.entries);
-        ZK_CHECK(cudaGetLastError());
-        if (needs_phi(p)) msm_phi_kernel<<<nblk, tb, 0, st>>>(bases, p.n, s.phi);
+                                                      s.entries, bases, s.phi);
     } else {
         msm_scatter_kernel<false><<<nblk, tb, 0, st>>>(scalars, p.n, p.c, p.W, kw, pw, phi_off, s.offset, s.count,
-                                                       s.entries);
+                                                       s.entries, nullptr, nullptr);
     }
     ZK_CHECK(cudaGetLastError());
     msm_accumulate_kernel<<<(p.nacc + 127) / 128, 128, 0, st>>>(s.entries, s.offset, p.NB, bases, s.phi,
