@@ -159,20 +159,33 @@ struct DftK {
     __device__ __forceinline__ typename TW::K w4() const { return TW::sm(k); }
     __device__ __forceinline__ typename TW::K cu() const { return TW::sm(k + TW::EW); }
     __device__ __forceinline__ typename TW::K su() const { return TW::sm(k + 2 * TW::EW); }
+    // Made by threads 0 to 2 of a block in two steps, the loads before the block's
+    // tile is read and the rest after, so that one wait covers both.
     // tw: the table of w_n, n = 2^log_n >= 8
-    __device__ __forceinline__ void init(const Fr* tw, int log_n) {
-        for (int i = threadIdx.x; i < 3; i += blockDim.x) {
-            typename TW::K r;
-            if (i == 0) {
-                r = TW::ld(tw, (size_t)1 << (log_n - 2));
-            } else {
-                const Fr a = TW::ld(tw, (size_t)1 << (log_n - 3)).w, b = TW::ld(tw, (size_t)3 << (log_n - 3)).w;
-                Fr h = i == 1 ? fe_sub<FrCfg>(a, b) : fe_add<FrCfg>(a, b);
-                limbs_half_mod<FrCfg>(h.v);
-                r = TW::of(h);
-            }
-            TW::put(k + i * TW::EW, r);
+    struct Raw {
+        typename TW::K a;
+        Fr b;
+    };
+    static __device__ __forceinline__ Raw fetch(int i, const Fr* tw, int log_n) {
+        Raw r;
+        if (i < 3) {
+            r.a = TW::ld(tw, (size_t)1 << (log_n - (i ? 3 : 2)));
+            r.b = TW::ld(tw, (size_t)3 << (log_n - 3)).w;
         }
+        return r;
+    }
+    __device__ __forceinline__ void put(int i, const Raw& r) {
+        if (i >= 3) return;
+        typename TW::K f = r.a;
+        if (i) {
+            Fr h = i == 1 ? fe_sub<FrCfg>(r.a.w, r.b) : fe_add<FrCfg>(r.a.w, r.b);
+            limbs_half_mod<FrCfg>(h.v);
+            f = TW::of(h);
+        }
+        TW::put(k + i * TW::EW, f);
+    }
+    __device__ __forceinline__ void init(const Fr* tw, int log_n) {
+        for (int i = threadIdx.x; i < 3; i += blockDim.x) put(i, fetch(i, tw, log_n));
     }
 };
 
@@ -404,7 +417,19 @@ ntt_pass_kernel(NttPassArgs a) {
     __shared__ Fr kst[G * 8 * TW::EW];
     __shared__ DftK<TW> dk;
     const bool kst_used = a.scale && !a.in_mul;
-    dk.init(a.tw, a.log_n);
+    typename DftK<TW>::Raw dk_raw;
+    if (T >= 3) dk_raw = DftK<TW>::fetch(tid, a.tw, a.log_n);
+    // coalesced load: chunk c -> (i, g, h); global x[q0 + g + (i << log_items)]
+    for (int c = tid; c < G * R * 2; c += T) {
+        const int h = c & 1, e = c >> 1;
+        const int g = e % G, i = e / G;
+        const size_t gi = (size_t)(q0 + g) + ((size_t)i << log_items);
+        *sm_slot(sm + g * R, i, h) = reinterpret_cast<const uint4*>(src + gi)[h];
+    }
+    if (T >= 3)
+        dk.put(tid, dk_raw);
+    else
+        dk.init(a.tw, a.log_n);
     if (kst_used) {
         for (int k = tid; k < G * 8; k += T) {
             const uint32_t qk = q0 + k / 8, i = k % 8;
@@ -413,13 +438,6 @@ ntt_pass_kernel(NttPassArgs a) {
             if (i * J) f = TW::prod(TW::ld(a.tw, (size_t)(i * J) << (a.log_n - a.log_p - 3)), f);
             TW::put(kst + k * TW::EW, f);
         }
-    }
-    // coalesced load: chunk c -> (i, g, h); global x[q0 + g + (i << log_items)]
-    for (int c = tid; c < G * R * 2; c += T) {
-        const int h = c & 1, e = c >> 1;
-        const int g = e % G, i = e / G;
-        const size_t gi = (size_t)(q0 + g) + ((size_t)i << log_items);
-        *sm_slot(sm + g * R, i, h) = reinterpret_cast<const uint4*>(src + gi)[h];
     }
     __syncthreads();
 
