@@ -332,7 +332,8 @@ cudaError_t zkp_extend_batch_tables(void *ext_out, void *coeff_out, const void *
 /* out[i] = (accumulate ? out[i] : 0) + 1 / (in[i] + c[0]) (c may be NULL);
  * zero maps to zero. out may alias in.  scratch: NULL or
  * zkp_scan_scratch_elems(n) device elements (not aliasing out or in); with it
- * the whole array takes one field inversion instead of one per 2048 elements. */
+ * arrays above 2^22 elements take one field inversion in all, else one is taken
+ * per 512, 1024 or 2048 elements. */
 cudaError_t zkp_batch_inverse(void *out, const void *in, const void *c, uint32_t n, int accumulate, void *scratch,
                               cudaStream_t stream);
 

@@ -36,7 +36,7 @@ def test_batch_inverse(O, gpu, n, with_scratch):
 
 
 # around the sizes where a thread takes 2, 4 and 8 elements
-@pytest.mark.parametrize("n", [511, 512, 513, 151552, 151553, 303104, 303105])
+@pytest.mark.parametrize("n", [511, 512, 513, 151552, 151553, 303104, 303105, 1212416, 1212417])
 def test_batch_inverse_elements_per_thread(O, gpu, n):
     H = gpu.host
     a = O.rand_fr(n, 300 + n % 997)

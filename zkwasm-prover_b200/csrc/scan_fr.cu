@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(ST) batch_prod_kernel(Src src, uint32_t n, Fr*
 // K = 8 three blocks fit an SM.  The tree takes 36 products of whole warps a
 // block, where exclusive prefixes and suffixes of the chunk products by two
 // block scans took 176.  Bound by the chain of tree and inversion while it
-// waits (2^15 elements: 114 -> 30 us with K = 2; 2^20: 218 -> 116 us).
+// waits (2^15 elements: 114 -> 30 us with K = 2; 2^20: 218 -> 102 us with K = 4).
 template <int K>
 static constexpr size_t batch_inv_smem() {
     return (size_t)(K + 1) * ST * sizeof(Fr);
@@ -238,7 +238,8 @@ size_t batch_inv_scratch_elems(uint32_t n) {
 // inversion at the top), (3) every block unwound with its product's inverse.
 // Otherwise each block inverts its own product: the extra pass of
 // the three-phase form costs more than the inversions that other resident
-// blocks partly hide (measured before the division steps at 2^16 and 2^22).
+// blocks partly hide.  The line dates from slower inversions: with scratch 2^23
+// elements take 0.80 ms, 0.67 without.
 static constexpr uint32_t BATCH_INV_THREE_PHASE_ABOVE = 1u << 22;
 
 template <int K, class Src, class Dst>
@@ -262,11 +263,13 @@ static cudaError_t launch_batch_inv(Src src, Dst dst, uint32_t n, Fr* scratch, s
                                   scratch_elems - 2 * (size_t)nb, s));
         return launch_batch_inv_k<SK>(src, dst, n, inv, s);
     }
-    // elements a thread: eight once that fills the SMs twice over, fewer below,
-    // where a block's chain of dependent products is the time (2^15 elements:
-    // 16 blocks at eight, 64 at two)
-    if (n > 4 * 2 * 148 * ST) return launch_batch_inv_k<8>(src, dst, n, nullptr, s);
-    if (n > 2 * 2 * 148 * ST) return launch_batch_inv_k<4>(src, dst, n, nullptr, s);
+    // Elements a thread: two where that makes up to four blocks an SM, four where
+    // that makes up to eight, else eight.  Short arrays pay for a block's chain of
+    // dependent products, long ones for the blocks' inversions (2, 4, 8 elements:
+    // 2^16 29.8, 35.0, 45.2 us; 303104 41.1, 43.1, 45.2; 303105 64.3, 49.3, 56.5;
+    // 2^20 142, 102, 113; 1.5 million 188, 135, 129).
+    if (n > 4 * 8 * 148 * ST) return launch_batch_inv_k<8>(src, dst, n, nullptr, s);
+    if (n > 2 * 4 * 148 * ST) return launch_batch_inv_k<4>(src, dst, n, nullptr, s);
     return launch_batch_inv_k<2>(src, dst, n, nullptr, s);
 }
 

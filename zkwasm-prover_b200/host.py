@@ -370,7 +370,7 @@ def scan_scratch(n: int) -> torch.Tensor:
 
 def batch_inverse(out, inp, c=None, accumulate=False, scratch=None, stream=None):
     """out = (accumulate ? out : 0) + 1 / (inp + c); scratch from scan_scratch(n)
-    (or None for one field inversion per 2048 elements)."""
+    (or None: one field inversion per 512 to 2048 elements at any n)."""
     abi.check(lib().zkp_batch_inverse(ptr(out), ptr(inp), ptr(c), inp.shape[0], int(accumulate), ptr(scratch),
                                       stream_handle(stream)), "zkp_batch_inverse")
 
