@@ -107,6 +107,20 @@ void hc_xyzz_add(uint64_t* out, const uint64_t* p, const uint64_t* q) { stx(out,
 
 void hc_xyzz_dbl(uint64_t* out, const uint64_t* p) { stx(out, xyzz_dbl(ldx(p))); }
 
+// [k] p for a small unsigned k (double-and-add from the top bit)
+static Xyzz xyzz_mul_u32(const Xyzz& p, uint32_t k) {
+    Xyzz r = xyzz_identity();
+    if (k == 0 || xyzz_is_id(p)) return r;
+    int top = 31;
+    while (!((k >> top) & 1)) top--;
+    r = p;
+    for (int b = top - 1; b >= 0; b--) {
+        r = xyzz_dbl(r);
+        if ((k >> b) & 1) r = xyzz_add(r, p);
+    }
+    return r;
+}
+
 void hc_xyzz_mul_u32(uint64_t* out, const uint64_t* p, uint32_t k) { stx(out, xyzz_mul_u32(ldx(p), k)); }
 
 void hc_xyzz_to_jac(uint64_t* out, const uint64_t* p) {

@@ -260,20 +260,6 @@ ZK_HD Xyzz xyzz_add(const Xyzz& p, const Xyzz& q) {
     return r;
 }
 
-// [k] p for a small unsigned k (double-and-add from the top bit)
-ZK_HD Xyzz xyzz_mul_u32(const Xyzz& p, uint32_t k) {
-    Xyzz r = xyzz_identity();
-    if (k == 0 || xyzz_is_id(p)) return r;
-    int top = 31;
-    while (!((k >> top) & 1)) top--;
-    r = p;
-    for (int b = top - 1; b >= 0; b--) {
-        r = xyzz_dbl(r);
-        if ((k >> b) & 1) r = xyzz_add(r, p);
-    }
-    return r;
-}
-
 // XYZZ -> Jacobian without an inversion: with ZZ = z^2, ZZZ = z^3 the point
 // (X * ZZ^2, Y * ZZ^3, ZZZ) has X'/Z'^2 = X/ZZ and Y'/Z'^3 = Y/ZZZ.
 // The identity becomes (0, 1, 0), halo2's Jacobian identity.

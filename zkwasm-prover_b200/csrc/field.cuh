@@ -822,15 +822,18 @@ ZK_HD void limbs_half_mod(uint32_t x[8]) {
 // ---------------------------------------------------------------------------
 // Inverse by division steps (D. J. Bernstein and B.-Y. Yang, "Fast
 // constant-time gcd computation and modular inversion", 2019), in the variant
-// that starts at delta = 1/2.  A step takes (delta, f, g), f odd, to
+// that starts at delta = 1/2 (P. Wuille, G. Maxwell, "safegcd implementation",
+// the notes of libsecp256k1, 2021).  A step takes (delta, f, g), f odd, to
 //     (1 - delta, g, (g - f) / 2)              if delta > 0 and g is odd,
 //     (1 + delta, f, (g + (g mod 2) f) / 2)    otherwise,
 // and from f = m, g = a it reaches g = 0, f = +-1.  Thirty steps look at the
 // lowest 30 bits of f and g only, so they run on two words and are collected in
 // a matrix of 31-bit entries that is then applied to the long f, g and to the
 // cofactors d, e (f = d a, g = e a mod m, each application an exact division by
-// 2^30 after adding the multiple of m that makes it one).  At most 590 steps
-// for 256-bit m; the loop ends when g is zero.
+// 2^30 after adding the multiple of m that makes it one).  The loop ends when g
+// is zero; its 600 steps cover the bound of those notes, 590 from delta = 1/2 for
+// 0 <= g <= f < 2^256 (by convex hulls of the reachable (f, g)), so a has to be
+// below m.
 //
 // Numbers are nine limbs of 30 bits, the top one signed.  Against the binary
 // Euclid it replaces, one bit of 8-limb chains at a time, a step is a few

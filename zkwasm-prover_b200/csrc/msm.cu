@@ -438,7 +438,8 @@ __device__ __forceinline__ void st_aff(Aff* p, const Aff& a) {
 // own windows): window j's XYZZ form is parked in its two table slots (X, Y in
 // the base's slot, ZZ, ZZZ in the image's), the product of the ZZ ZZZ is
 // inverted once, and the windows are converted from the last back.  An
-// inversion is about 36 us of one thread, so W - 1 of them dominated the build.
+// inversion is about 20 us of one thread, W - 1 of them would be most of the
+// build.
 __global__ void __launch_bounds__(128) msm_table_kernel(Aff* __restrict__ table, const Aff* __restrict__ bases,
                                                         uint32_t nsrs, int c, int W) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -515,7 +516,8 @@ static int pick_c(uint32_t n, bool glv) {
 // over a table: every window's digits go into one bucket set, so the
 // reduction is paid once and there is no Horner chain.  A bucket costs about
 // five sorted entries (its reduction and the shorter runs of a wider key
-// space), fitted to B200 timings at 2^14..2^22 points.
+// space), fitted to B200 timings at 2^14..2^22 points (before the reduction's
+// tree).
 static int pick_c_table(uint32_t n) {
     int best = 4;
     double best_cost = 1e300;
@@ -532,9 +534,10 @@ static int pick_c_table(uint32_t n) {
 int msm_table_default_window(uint32_t n) { return pick_c_table(n); }
 
 // one width for a batch over one table: each MSM has its own bucket set, and
-// with many sets in one pipeline a bucket costs about 25 sorted entries (their
-// reductions share one thread budget), fitted to 256 MSMs of 2^14..2^22
-// points on B200 (c = 13..17: 456, 450, 431, 413, 429 ms; 19: 525 ms)
+// with many sets in one pipeline a bucket costs about 25 sorted entries.  Fitted
+// to 256 MSMs of 2^14..2^22 points on B200 (c = 13..17: 456, 450, 431, 413, 429
+// ms; 19: 525 ms) with a reduction that cost more a bucket than the present
+// tree (384 ms at 16).
 int msm_batch_table_default_window(const uint32_t* n, uint32_t count) {
     double pts = 0;
     for (uint32_t i = 0; i < count; i++) pts += 2.0 * n[i];

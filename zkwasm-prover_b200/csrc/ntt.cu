@@ -58,13 +58,10 @@ __device__ __noinline__ Fr nt_mulz(const Fr a, const Fr b) { return fe_mul_lazy<
 __device__ __noinline__ Fr nt_shoup(const Fr a, const Fr w, const Fr wp) { return fe_mul_shoup<FrCfg>(a, w, wp); }
 #endif
 
-// Two or three independent products in one call, so the scheduler can
-// interleave their carry chains.
+// Two independent products in one call, so the scheduler can interleave their
+// carry chains.
 struct Fr2 {
     Fr a, b;
-};
-struct Fr3 {
-    Fr a, b, c;
 };
 #if defined(ZK_NTT_INLINE_MUL)
 #define ZK_NTMUL __device__ __forceinline__
@@ -74,15 +71,8 @@ struct Fr3 {
 ZK_NTMUL Fr2 nt_mulz2(const Fr a0, const Fr w0, const Fr a1, const Fr w1) {
     return {fe_mul_lazy<FrCfg>(a0, w0), fe_mul_lazy<FrCfg>(a1, w1)};
 }
-ZK_NTMUL Fr3 nt_mulz3(const Fr a0, const Fr w0, const Fr a1, const Fr w1, const Fr a2, const Fr w2) {
-    return {fe_mul_lazy<FrCfg>(a0, w0), fe_mul_lazy<FrCfg>(a1, w1), fe_mul_lazy<FrCfg>(a2, w2)};
-}
 ZK_NTMUL Fr2 nt_shoup2(const Fr a0, const Fr w0, const Fr p0, const Fr a1, const Fr w1, const Fr p1) {
     return {fe_mul_shoup<FrCfg>(a0, w0, p0), fe_mul_shoup<FrCfg>(a1, w1, p1)};
-}
-ZK_NTMUL Fr3 nt_shoup3(const Fr a0, const Fr w0, const Fr p0, const Fr a1, const Fr w1, const Fr p1, const Fr a2,
-                       const Fr w2, const Fr p2) {
-    return {fe_mul_shoup<FrCfg>(a0, w0, p0), fe_mul_shoup<FrCfg>(a1, w1, p1), fe_mul_shoup<FrCfg>(a2, w2, p2)};
 }
 #undef ZK_NTMUL
 
@@ -99,10 +89,6 @@ struct TwM {
     static __device__ __forceinline__ Fr mul(const Fr& v, const K& k) { return nt_mulz(v, k.w); }
     static __device__ __forceinline__ Fr2 mul2(const Fr& v0, const K& k0, const Fr& v1, const K& k1) {
         return nt_mulz2(v0, k0.w, v1, k1.w);
-    }
-    static __device__ __forceinline__ Fr3 mul3(const Fr& v0, const K& k0, const Fr& v1, const K& k1, const Fr& v2,
-                                               const K& k2) {
-        return nt_mulz3(v0, k0.w, v1, k1.w, v2, k2.w);
     }
     static __host__ __device__ __forceinline__ const Fr* off(const Fr* t, size_t i) { return t + i; }
     static constexpr int EW = 1;  // elements an entry
@@ -122,10 +108,6 @@ struct TwS {
     static __device__ __forceinline__ Fr mul(const Fr& v, const K& k) { return nt_shoup(v, k.w, k.wp); }
     static __device__ __forceinline__ Fr2 mul2(const Fr& v0, const K& k0, const Fr& v1, const K& k1) {
         return nt_shoup2(v0, k0.w, k0.wp, v1, k1.w, k1.wp);
-    }
-    static __device__ __forceinline__ Fr3 mul3(const Fr& v0, const K& k0, const Fr& v1, const K& k1, const Fr& v2,
-                                               const K& k2) {
-        return nt_shoup3(v0, k0.w, k0.wp, v1, k1.w, k1.wp, v2, k2.w, k2.wp);
     }
     static __host__ __device__ __forceinline__ const Fr* off(const Fr* t, size_t i) { return t + 2 * i; }
     static constexpr int EW = 2;
@@ -889,8 +871,9 @@ cudaError_t ntt_pass(const NttPassArgs& a, int log_r, unsigned ny, unsigned nz, 
 #define ZK_NTT_MAX_PASS_BITS 11
 #endif
 // The splits the radix autotuner (zkp_ntt_batch_plan over every split into
-// 2-3 passes of 2^6..2^12, one column) measured fastest on B200 for 2^13..2^25;
-// other sizes use the even split below.
+// 2-3 passes of 2^6..2^12, one column) measured fastest on B200 for 2^13..2^25,
+// with passes whose twiddles came after the DFT; other sizes use the even split
+// below, columns of up to NTT_SHORT elements in all two even passes (ntt_run).
 static const int8_t TUNED_SPLIT[13][3] = {{7, 6, 0},  {6, 8, 0},  {6, 9, 0},   {8, 8, 0},  {8, 9, 0},
                                           {9, 9, 0},  {11, 8, 0}, {10, 10, 0}, {11, 10, 0}, {11, 11, 0},
                                           {11, 6, 6}, {9, 9, 6},  {9, 10, 6}};
