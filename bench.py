@@ -136,6 +136,18 @@ class ClockSampler:
 # ------------------------------------------------------------------ workload
 
 
+# Products per element of a pass's first radix-8 sub-stage: four in the DFT of
+# eight, and before it none (a first pass), seven (twiddles) or eight (a scale, a
+# coset's shift, a factor per input)
+FIRST_PLAIN, FIRST_TWIDDLES, FIRST_SCALED = 4 / 8, 11 / 8, 12 / 8
+
+
+def pass_products(log_r, first):
+    """Fr products per element of one transform pass of radix 2^log_r: radix-8
+    sub-stages, then a radix-4 (one product an element) or radix-2 (a half)."""
+    return first + 11 / 8 * (log_r // 3 - 1) + (0, 1 / 2, 1)[log_r % 3]
+
+
 class ExtendPhase:
     """64 columns: iNTT 2^log_n -> coset NTT on 2^(log_n + ext_bits)."""
 
@@ -166,9 +178,7 @@ class ExtendPhase:
         return (3 + self.E) * self.n * 32
 
     def mults_per_column(self):
-        n, lg, E = self.n, self.log_n, self.E
-        ntt = (n // 2) * lg
-        return ntt + n + E * (ntt + n)  # iNTT + n^-1 scale, E sub-transforms + twist
+        return sum(self.stage_mults()) / self.chunk
 
     def fused(self):
         """zkp_extend_batch fuses the last inverse pass with the first coset
@@ -189,14 +199,18 @@ class ExtendPhase:
         return [2 * c * n * 32, 2 * c * n * 32, (2 + E) * c * n * 32, 2 * E * c * n * 32]
 
     def stage_mults(self):
-        """algorithmic Fr products per stage launch: (n/2) log2 n per
-        transform split evenly over its two passes, n for the n^-1 scale and n
-        for each coset twist."""
-        c, n, E, lg = self.chunk, self.n, self.E, self.log_n
-        half = (n // 2) * lg // 2
+        """Fr products per stage launch: the passes' (pass_products) over the
+        even split, the n^-1 scale in the inverse transform's last pass and a
+        coset's shift in its first."""
+        c, n, E = self.chunk, self.n, self.E
+        r0, r1 = (self.log_n + 1) // 2, self.log_n // 2
+        inv0, inv1 = pass_products(r0, FIRST_PLAIN), pass_products(r1, FIRST_SCALED)
+        # the fused stage's cosets start from the radix of its inverse pass
+        f0, f1 = (r1, r0) if self.fused() else (r0, r1)
+        cos0, cos1 = pass_products(f0, FIRST_SCALED), pass_products(f1, FIRST_TWIDDLES)
         if self.fused():
-            return [c * half, 0, c * (half + n + E * (half + n)), c * E * half]
-        return [c * half, c * (half + n), c * E * (half + n), c * E * half]
+            return [c * n * inv0, 0, c * n * (inv1 + E * cos0), c * n * E * cos1]
+        return [c * n * inv0, c * n * inv1, c * n * E * cos0, c * n * E * cos1]
 
     def launches_per_step(self):
         return (self.C // self.chunk) * 4
@@ -482,7 +496,12 @@ def run_rows(lib, device, mont_rate, peak_hbm, ours=True, log_n=22, log_ext=24, 
         buf = random_fr(nt, 1300 + log_nt, device)
         tmp = torch.empty_like(buf)
         swap = ctypes.c_bool(False)
-        return (f"a6 ntt (one column, 2^{log_nt})", 2 * nt * E, (nt // 2) * log_nt, "ntt",
+        mults = (nt // 2) * log_nt  # radix 2
+        if ours:
+            rad = (ctypes.c_int * 4)()
+            passes = rad[:lib.zkp_ntt_default_plan(log_nt, ctypes.addressof(rad))]
+            mults = nt * sum(pass_products(r, FIRST_TWIDDLES if i else FIRST_PLAIN) for i, r in enumerate(passes))
+        return (f"a6 ntt (one column, 2^{log_nt})", 2 * nt * E, mults, "ntt",
                 [(P, buf), (P, tmp), (P, pq), (P, om), (P, None), (I, log_nt), (I, 8), ("hostptr", swap), (S, st)],
                 True), (om, pq, buf, tmp, swap)
 
@@ -1493,12 +1512,14 @@ def run_pipeline(args):
         mont_rate = calib_mont_rate(zkp, device)
         # per launch group: read 32 coefficient columns, write 32 coset columns
         # (algorithmic bytes; the intermediate pass round trip is not counted),
-        # (n/2) log n butterfly products + n twist products per column
+        # and the products its passes make, the coset's factors in the first
         groups = len(timed)
         avg_ms = ntt_ms / max(1, groups)
         cols_per = ntt_cols / max(1, groups)
         bytes_per = cols_per * 2 * n * 32
-        mults_per = cols_per * (n // 2 * shape.k + n)
+        radices = zkp.host.ntt_default_plan(shape.k)
+        mults_per = cols_per * n * sum(pass_products(r, FIRST_TWIDDLES if i else FIRST_SCALED)
+                                       for i, r in enumerate(radices))
         achieved = bytes_per / (avg_ms / 1e3) / 1e9
         extra = {}
         if ws == 1 and not args.no_extras:

@@ -132,9 +132,12 @@ def test_ntt_short_passes(O, gpu, log_n, ncols):
     assert (H.to_host(out) == a).all()
 
 
-# fused stage radices: 2^18 -> 2^9, 2^19 -> 2^9, 2^20 and 2^21 -> 2^10, 2^22 -> 2^11
+# fused stage radices: 2^18 -> 2^9, 2^19 -> 2^9, 2^20 and 2^21 -> 2^10, 2^22 -> 2^11;
+# 2^7 to 2^14: one and two passes through the short kernel (all cosets' columns
+# up to 2^16 elements) and, for the pairs, beside it; one and sixteen cosets
 @pytest.mark.parametrize("pairs", [False, True])
-@pytest.mark.parametrize("log_n,ext_bits,ncols", [(4, 3, 2), (10, 3, 3), (13, 3, 2), (16, 2, 2),
+@pytest.mark.parametrize("log_n,ext_bits,ncols", [(4, 3, 2), (7, 3, 1), (8, 2, 3), (9, 3, 2), (10, 3, 3), (13, 3, 1),
+                                                  (13, 3, 2), (14, 2, 1), (16, 2, 2), (18, 0, 2), (18, 4, 1),
                                                   (18, 3, 2), (19, 2, 1), (20, 3, 1), (22, 1, 1)])
 def test_extend_batch_matches_coset_ntt(O, gpu, log_n, ext_bits, ncols, pairs):
     # pairs: the same phase over (w, w') tables and products by known factors
